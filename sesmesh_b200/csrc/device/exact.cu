@@ -1058,6 +1058,72 @@ __global__ void __launch_bounds__(32 * X_WARPS, 4) k_refine_exact(DArr A, DLat L
     }
 }
 
+// A block of T threads per entry: the entry's ball in `region` bytes of the
+// block's shared memory, built by all threads, then its edges by groups of RG
+// lanes.  MARKED = false: an entry is a work item (list[q]; null: every
+// item) and each group takes every (T / RG)-th of its edges.  MARKED = true:
+// an entry is one edge, refined by the block's first group.  n_dev (or
+// n_host, when null) entries are claimed from *queue; those whose lists do
+// not fit go to ovf (ovf[0] = count, then the entries).
+// Bound by f64 latency (dependent square roots, divisions and shared-memory
+// loads): 16 warps to an SM at 128 registers, 32 at 64 (some spills, which
+// the longer lists' walks repay).  16 lanes per edge against 32 on lists of
+// 13 KB: 30.2 against 30.9 ms (106,539 sub-blocks); 32 lanes and one
+// 512-thread block where a block's lists take the whole shared memory:
+// 511.5 ms (shell of 2.4 M spheres at 1 A), 742.7 ms with 256 threads, 583 ms
+// by warps and slabs.
+template <bool MARKED, int RG, int T, int MB>
+__global__ void __launch_bounds__(T, MB) k_refine_exact_block(
+    DArr A, DLat L, ExactAttr X, const int4* keys, const uint32_t* work, const uint32_t* edges,
+    const float2* edge_vals, const uint32_t* item_off, const uint32_t* item_edges, const uint32_t* edge_off,
+    uint32_t n_bricks, const uint32_t* list, const uint32_t* n_dev, uint32_t n_host, ExactOut out, size_t region,
+    uint32_t* ovf, unsigned int* queue, const uint32_t* rec, int slack, const uint32_t* gids, const uint8_t* window) {
+    extern __shared__ __align__(16) unsigned char xs[];
+    __shared__ uint32_t cnt[8];
+    __shared__ uint32_t sh_q;
+    const uint32_t tid = threadIdx.x;
+    const uint32_t n_claim = n_dev ? *n_dev : n_host;
+    for (;;) {
+        __syncthreads();  // the previous entry's lists are no longer read
+        if (tid == 0) sh_q = atomicAdd(queue, 1u);
+        __syncthreads();
+        const uint32_t q = sh_q;
+        if (q >= n_claim) break;
+        const uint32_t i = list ? list[q] : q;
+        uint32_t a0 = 0, a1 = 1, j;
+        if (MARKED) {
+            uint32_t lo = 0, hi = n_bricks;  // the brick of edge i: edge_off[lo] <= i < edge_off[lo + 1]
+            while (hi - lo > 1) {
+                const uint32_t mid = (lo + hi) >> 1;
+                if (edge_off[mid] <= i) lo = mid;
+                else hi = mid;
+            }
+            const uint32_t b = uint32_t(L.b), sub = uint32_t(L.sub), cell = edges[i] / 3;
+            j = 8 * lo + min(cell % b / sub, 1u) + 2 * min(cell / b % b / sub, 1u) + 4 * min(cell / (b * b) / sub, 1u);
+            // As k_item_edges: edges of sub-blocks that were not sampled
+            // stay with the host.
+            if (rec[size_t(j) * REC_WORDS + R_STATE] != ST_SAMPLE) continue;
+        } else {
+            a0 = item_off[i], a1 = item_off[i + 1];
+            if (a0 == a1) continue;
+            j = work[i];
+        }
+        const int4 key = keys[j >> 3];
+        XView v;
+        if (!x_ball<true>(A, L, key, j, xs, region, cnt, tid, T, v, slack >= 0 ? rec + size_t(j) * REC_WORDS : nullptr,
+                          slack, gids, window)) {
+            if (tid == 0) ovf[1 + atomicAdd(&ovf[0], 1u)] = i;
+            continue;
+        }
+        const uint32_t lane = tid & 31;
+        const uint32_t gm = (0xffffffffu >> (32 - RG)) << (lane & ~uint32_t(RG - 1));
+        for (uint32_t e = a0 + tid / RG; e < a1; e += T / RG) {
+            const uint32_t k = MARKED ? i : item_edges[e];
+            x_edge<false, RG>(v, A, L, X, key, k, edges[k], edge_vals[k], out, nullptr, int(lane % RG), gm);
+        }
+    }
+}
+
 // Sum of the edges' evaluation counts and the number of edges left to the
 // host (evals = 0): out[0], out[1].
 __global__ void k_exact_summary(const uint32_t* evals, size_t n, unsigned long long* out) {
@@ -1081,13 +1147,13 @@ __global__ void k_exact_summary(const uint32_t* evals, size_t n, unsigned long l
 // refinement converged on (t in [0, 1], a valid feature) is placed at
 // pa + d clamp(t) with the exact attributes of its feature and closest
 // point (brick origin + the f32 offset); every other edge is marked in
-// need[] for the exact refinement.  counters[0] += the marked edges.
+// need[] and listed (in no order) for the exact refinement, *marked counting
+// them.
 __global__ void k_place_fast(DArr A, DLat L, ExactAttr X, const int4* keys, uint32_t n_bricks,
                              const uint32_t* edge_off, const uint32_t* edges, const float2* edge_vals, size_t n_edges,
                              const float* t_in, const uint32_t* feat, const float* q, const uint32_t* ev_in,
-                             ExactOut out, uint8_t* need, unsigned long long* marked) {
+                             ExactOut out, uint8_t* need, uint32_t* list, unsigned long long* marked) {
     const size_t k = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
-    unsigned long long mine = 0;
     if (k < n_edges) {
         const uint32_t ev = ev_in[k];
         const double t = double(t_in[k]);
@@ -1102,7 +1168,7 @@ __global__ void k_place_fast(DArr A, DLat L, ExactAttr X, const int4* keys, uint
         if (!ok) {
             need[k] = 1;
             out.evals[k] = 0;
-            mine = 1;
+            list[atomicAdd(marked, 1ull)] = uint32_t(k);
         } else {
             need[k] = 0;
             uint32_t lo = 0, hi = n_bricks;  // the brick of edge k: edge_off[lo] <= k < edge_off[lo + 1]
@@ -1138,8 +1204,6 @@ __global__ void k_place_fast(DArr A, DLat L, ExactAttr X, const int4* keys, uint
             out.evals[k] = ev & 0x7fffffffu;
         }
     }
-    for (int o = 16; o; o >>= 1) mine += __shfl_down_sync(0xffffffffu, mine, o);
-    if ((threadIdx.x & 31) == 0 && mine) atomicAdd(marked, mine);
 }
 
 }  // namespace
@@ -1147,12 +1211,13 @@ __global__ void k_place_fast(DArr A, DLat L, ExactAttr X, const int4* keys, uint
 cudaError_t launch_place_fast(const DArr& A, const DLat& L, const ExactAttr& X, const int4* keys, uint32_t n_bricks,
                               const uint32_t* edge_off, const uint32_t* edges, const float2* edge_vals, size_t n_edges,
                               const float* t, const uint32_t* feat, const float* q, const uint32_t* evals,
-                              const ExactOut& out, uint8_t* need, unsigned long long* marked, cudaStream_t s) {
+                              const ExactOut& out, uint8_t* need, uint32_t* list, unsigned long long* marked,
+                              cudaStream_t s) {
     cudaError_t e = cudaMemsetAsync(marked, 0, 8, s);
     if (e != cudaSuccess || !n_edges) return e;
     count_launches(1);
     k_place_fast<<<unsigned((n_edges + 255) / 256), 256, 0, s>>>(A, L, X, keys, n_bricks, edge_off, edges, edge_vals,
-                                                                  n_edges, t, feat, q, evals, out, need, marked);
+                                                                  n_edges, t, feat, q, evals, out, need, list, marked);
     return cudaGetLastError();
 }
 
@@ -1165,14 +1230,39 @@ cudaError_t launch_exact_summary(const uint32_t* evals, size_t n, unsigned long 
     return cudaGetLastError();
 }
 
-template <bool COUNT, int RG, int RGS>
-static cudaError_t launch_exact_levels(const DArr& A, const DLat& L, const ExactAttr& X, const int4* keys,
-                                       const uint32_t* work, const uint32_t* edges, const float2* edge_vals,
-                                       const uint32_t* item_off, const uint32_t* item_edges, uint32_t n_items,
-                                       const ExactOut& out, uint32_t* ovf, unsigned char* slab, size_t slab_bytes,
-                                       unsigned long long* counters, int sms, size_t region, cudaStream_t s,
-                                       const uint32_t* rec, int slack, const uint32_t* gids,
-                                       const uint8_t* window);
+// List-size slack of a hint mode (smb_batch_set_exact_hint); -1: no hint.
+static int exact_slack(int hint) { return hint == 0 ? -1 : (hint == 2 ? 0 : X_HINT_SLACK); }
+
+template <bool MARKED, int RG, int T, int MB>
+static cudaError_t launch_block_one(const ExactBlock& B, const DArr& A, const DLat& L, const ExactAttr& X,
+                                    const ExactOut& out, int sms, cudaStream_t s) {
+    auto k = k_refine_exact_block<MARKED, RG, T, MB>;
+    cudaError_t e;
+    if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(B.region))) != cudaSuccess)
+        return e;
+    int per_sm = 0;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, T, B.region)) != cudaSuccess) return e;
+    if (per_sm < 1) return cudaErrorInvalidConfiguration;
+    const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>(B.n_max, uint32_t(sms * per_sm)));
+    count_launches(1);
+    k<<<grid, T, B.region, s>>>(A, L, X, B.keys, B.work, B.edges, B.edge_vals, B.item_off, B.item_edges, B.edge_off,
+                                B.n_bricks, B.list, B.n_dev, B.n_max, out, B.region, B.ovf,
+                                reinterpret_cast<unsigned int*>(B.queue), B.rec, exact_slack(B.hint), B.gids, B.window);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_refine_exact_block(const ExactBlock& B, const DArr& A, const DLat& L, const ExactAttr& X,
+                                      const ExactOut& out, int sms, cudaStream_t s) {
+    cudaError_t e;
+    if ((e = cudaMemsetAsync(B.queue, 0, 8, s)) != cudaSuccess || (e = cudaMemsetAsync(B.ovf, 0, 4, s)) != cudaSuccess)
+        return e;
+    if (!B.n_max) return cudaSuccess;
+    // One edge per block: a warp refines it, the others help build the lists.
+    if (B.marked) return launch_block_one<true, 32, 256, 2>(B, A, L, X, out, sms, s);
+    if (!B.wide) return launch_block_one<false, 8, 128, 4>(B, A, L, X, out, sms, s);
+    return B.region > BLOCK_HALF_SM ? launch_block_one<false, 32, 512, 1>(B, A, L, X, out, sms, s)
+                                    : launch_block_one<false, 16, 512, 2>(B, A, L, X, out, sms, s);
+}
 
 size_t exact_slab_bytes(int sms) {
     int per_sm = 0;
@@ -1180,70 +1270,56 @@ size_t exact_slab_bytes(int sms) {
     return size_t(std::max(sms, 1)) * size_t(std::max(per_sm, 1)) * X_WARPS * EXACT_SLAB;
 }
 
-cudaError_t launch_refine_exact(const DArr& A, const DLat& L, const ExactAttr& X, const int4* keys,
-                                const uint32_t* work, const uint32_t* edges, const float2* edge_vals,
-                                const uint32_t* item_off, const uint32_t* item_edges, uint32_t n_items,
-                                const ExactOut& out, uint32_t* ovf, unsigned char* slab, size_t slab_bytes,
-                                unsigned long long* counters, int sms, size_t region, cudaStream_t s, bool count,
-                                int group, const uint32_t* rec, int hint, const uint32_t* gids,
-                                const uint8_t* window) {
-    const int slack = hint == 2 ? 0 : X_HINT_SLACK;
-    if (hint == 0) rec = nullptr;
-    if (count) {
-        cudaError_t e = cudaMemsetAsync(&counters[CNT_OPS], 0, 8, s);
-        if (e != cudaSuccess) return e;
-        return launch_exact_levels<true, 1, 1>(A, L, X, keys, work, edges, edge_vals, item_off, item_edges,
-                                               n_items, out, ovf, slab, slab_bytes, counters, sms, region, s, rec, slack, gids, window);
-    }
-    // The slab pass takes the largest lists: at least 8 lanes per edge.
-    if (group == 32)
-        return launch_exact_levels<false, 32, 32>(A, L, X, keys, work, edges, edge_vals, item_off, item_edges,
-                                                  n_items, out, ovf, slab, slab_bytes, counters, sms, region, s, rec, slack, gids, window);
-    if (group == 8)
-        return launch_exact_levels<false, 8, 8>(A, L, X, keys, work, edges, edge_vals, item_off, item_edges, n_items,
-                                                out, ovf, slab, slab_bytes, counters, sms, region, s, rec, slack, gids, window);
-    return launch_exact_levels<false, 1, 8>(A, L, X, keys, work, edges, edge_vals, item_off, item_edges, n_items,
-                                            out, ovf, slab, slab_bytes, counters, sms, region, s, rec, slack, gids, window);
-}
-
-template <bool COUNT, int RG, int RGS>
-static cudaError_t launch_exact_levels(const DArr& A, const DLat& L, const ExactAttr& X, const int4* keys,
-                                       const uint32_t* work, const uint32_t* edges, const float2* edge_vals,
-                                       const uint32_t* item_off, const uint32_t* item_edges, uint32_t n_items,
-                                       const ExactOut& out, uint32_t* ovf, unsigned char* slab, size_t slab_bytes,
-                                       unsigned long long* counters, int sms, size_t region, cudaStream_t s,
-                                       const uint32_t* rec, int slack, const uint32_t* gids,
-                                       const uint8_t* window) {
+template <bool SLAB, bool COUNT, int RG>
+static cudaError_t launch_exact_warps(const ExactItems& I, const DArr& A, const DLat& L, const ExactAttr& X,
+                                      const ExactOut& out, int sms, cudaStream_t s) {
     cudaError_t e;
-    if ((e = cudaMemsetAsync(&counters[CNT_QUEUE], 0, 8, s)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(&counters[CNT_XQUEUE], 0, 8, s)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(ovf, 0, 8, s)) != cudaSuccess) return e;
-    if (!n_items) return cudaSuccess;
-    region = (region + 15) & ~size_t(15);
-    const size_t narrow = size_t(X_WARPS) * region;
-    auto kn = k_refine_exact<false, COUNT, RG>;
-    auto kg = k_refine_exact<true, COUNT, RGS>;
-    if ((e = cudaFuncSetAttribute(kn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(narrow))) != cudaSuccess)
-        return e;
-    int per_sm = 0;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kn, 32 * X_WARPS, narrow)) != cudaSuccess)
-        return e;
-    const uint32_t warps = (n_items + X_WARPS - 1) / X_WARPS;
-    const uint32_t grid = std::min<uint32_t>(warps, uint32_t(sms * std::max(per_sm, 1)));
-    count_launches(2);
+    auto k = k_refine_exact<SLAB, COUNT, RG>;
     // ovf[0]: items over the shared region, ovf[1..]: those items; the word
     // after the list counts the items over a slab (left to the host).
-    unsigned int* left = reinterpret_cast<unsigned int*>(ovf) + 1 + n_items;
-    if ((e = cudaMemsetAsync(left, 0, 4, s)) != cudaSuccess) return e;
-    kn<<<grid, 32 * X_WARPS, narrow, s>>>(A, L, X, keys, work, edges, edge_vals, item_off, item_edges, n_items, out,
-                                          region, ovf, nullptr, left, counters, rec, slack, gids, window);
-    // The overflowed items: a warp each, lists in a global slab.
-    const uint32_t slabs = uint32_t(slab_bytes / EXACT_SLAB);
-    const uint32_t grid_g = std::max<uint32_t>(1, slabs / X_WARPS);
-    if (!slab || !grid_g) return cudaErrorInvalidValue;
-    kg<<<grid_g, 32 * X_WARPS, 0, s>>>(A, L, X, keys, work, edges, edge_vals, item_off, item_edges, n_items, out,
-                                       EXACT_SLAB, ovf, slab, left, counters, rec, slack, gids, window);
+    unsigned int* left = reinterpret_cast<unsigned int*>(I.ovf) + 1 + I.n_items;
+    unsigned grid;
+    size_t smem = 0, region = EXACT_SLAB;
+    if (SLAB) {
+        grid = unsigned(I.slab_bytes / EXACT_SLAB / X_WARPS);
+        if (!I.slab || !grid) return cudaErrorInvalidValue;
+        if ((e = cudaMemsetAsync(&I.counters[CNT_XQUEUE], 0, 8, s)) != cudaSuccess) return e;
+        if ((e = cudaMemsetAsync(left, 0, 4, s)) != cudaSuccess) return e;
+    } else {
+        region = (I.region + 15) & ~size_t(15);
+        smem = size_t(X_WARPS) * region;
+        if ((e = cudaMemsetAsync(&I.counters[CNT_QUEUE], 0, 8, s)) != cudaSuccess) return e;
+        if ((e = cudaMemsetAsync(I.ovf, 0, 4, s)) != cudaSuccess) return e;
+        if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))) != cudaSuccess)
+            return e;
+        int per_sm = 0;
+        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 32 * X_WARPS, smem)) != cudaSuccess)
+            return e;
+        grid = std::min<unsigned>((I.n_items + X_WARPS - 1) / X_WARPS, unsigned(sms * std::max(per_sm, 1)));
+    }
+    if (!I.n_items) return cudaSuccess;
+    count_launches(1);
+    const int slack = exact_slack(I.hint);
+    k<<<grid, 32 * X_WARPS, smem, s>>>(A, L, X, I.keys, I.work, I.edges, I.edge_vals, I.item_off, I.item_edges,
+                                       I.n_items, out, region, I.ovf, SLAB ? I.slab : nullptr, left, I.counters,
+                                       slack < 0 ? nullptr : I.rec, slack, I.gids, I.window);
     return cudaGetLastError();
+}
+
+cudaError_t launch_refine_exact(const ExactItems& I, const DArr& A, const DLat& L, const ExactAttr& X,
+                                const ExactOut& out, int sms, cudaStream_t s) {
+    if (I.count) return launch_exact_warps<false, true, 1>(I, A, L, X, out, sms, s);
+    if (I.group == 32) return launch_exact_warps<false, false, 32>(I, A, L, X, out, sms, s);
+    if (I.group == 8) return launch_exact_warps<false, false, 8>(I, A, L, X, out, sms, s);
+    return launch_exact_warps<false, false, 1>(I, A, L, X, out, sms, s);
+}
+
+cudaError_t launch_refine_exact_slab(const ExactItems& I, const DArr& A, const DLat& L, const ExactAttr& X,
+                                     const ExactOut& out, int sms, cudaStream_t s) {
+    if (I.count) return launch_exact_warps<true, true, 1>(I, A, L, X, out, sms, s);
+    // The slab pass takes the largest lists: at least 8 lanes per edge.
+    if (I.group == 32) return launch_exact_warps<true, false, 32>(I, A, L, X, out, sms, s);
+    return launch_exact_warps<true, false, 8>(I, A, L, X, out, sms, s);
 }
 
 }  // namespace smb

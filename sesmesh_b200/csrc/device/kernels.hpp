@@ -147,32 +147,79 @@ struct ExactOut {
 };
 // Fast mode's placement on the device (mesh_brick_device, extract.rs:274-365):
 // converged edges placed with their exact attributes into out; need[k] = 1
-// (and *marked counts them) for the edges the exact refinement must take.
+// for the edges the exact refinement must take, which list gets (in no order,
+// *marked of them).
 cudaError_t launch_place_fast(const DArr& A, const DLat& L, const ExactAttr& X, const int4* keys, uint32_t n_bricks,
                               const uint32_t* edge_off, const uint32_t* edges, const float2* edge_vals, size_t n_edges,
                               const float* t, const uint32_t* feat, const float* q, const uint32_t* evals,
-                              const ExactOut& out, uint8_t* need, unsigned long long* marked, cudaStream_t s);
+                              const ExactOut& out, uint8_t* need, uint32_t* list, unsigned long long* marked,
+                              cudaStream_t s);
 // out[0] = sum of evals[0..n), out[1] = how many are 0.
 cudaError_t launch_exact_summary(const uint32_t* evals, size_t n, unsigned long long* out, int sms, cudaStream_t s);
-// f64 refinement of the work items' edge lists (k_item_edges): a warp per
-// item with `region` bytes of shared memory for the item's candidate lists,
-// then the items that did not fit with a warp each and a 256 KiB list slab
-// in global memory (slab: exact_slab_bytes(sms) bytes).  ovf: n_items + 2
+// f64 refinement of the work items' edge lists (k_item_edges).
+// launch_refine_exact: a warp per item with `region` bytes of shared memory
+// for the item's candidate lists; launch_refine_exact_slab: the items that
+// did not fit with a warp each and a 256 KiB list slab in global memory
+// (slab: exact_slab_bytes(sms) bytes).  ovf: n_items + 2
 // words (overflow count, items, then the count of items over a slab, whose
-// edges keep evals = 0).  count: counters[CNT_OPS] gets the f64 operations
-// of the field evaluations (x_eval's rules).  rec: the gather's records of
-// the sub-blocks (their list sizes bound each ball's), or null; hint 0: do
+// edges keep evals = 0).  count: counters[CNT_OPS] grows by the f64 operations
+// of the field evaluations (x_eval's rules).  group: lanes per edge (1, 8 or
+// 32; the slab pass at least 8).  rec: the gather's records of
+// the sub-blocks (their list sizes bound each ball's); hint 0: do
 // not use them, 2: bounds one short (every ball through the counted layout).
 // gids, window: the gather's candidate ids and its per-sub-block marks
 // (GatherOut::window); an unmarked sub-block takes its lists from the ids.
 size_t exact_slab_bytes(int sms);
-cudaError_t launch_refine_exact(const DArr& A, const DLat& L, const ExactAttr& X, const int4* keys,
-                                const uint32_t* work, const uint32_t* edges, const float2* edge_vals,
-                                const uint32_t* item_off, const uint32_t* item_edges, uint32_t n_items,
-                                const ExactOut& out, uint32_t* ovf, unsigned char* slab, size_t slab_bytes,
-                                unsigned long long* counters, int sms, size_t region, cudaStream_t s,
-                                bool count = false, int group = 1, const uint32_t* rec = nullptr, int hint = 1,
-                                const uint32_t* gids = nullptr, const uint8_t* window = nullptr);
+struct ExactItems {
+    const int4* keys;
+    const uint32_t *work, *edges;
+    const float2* edge_vals;
+    const uint32_t *item_off, *item_edges;
+    uint32_t n_items;
+    uint32_t* ovf;
+    unsigned char* slab;
+    size_t slab_bytes;
+    unsigned long long* counters;
+    size_t region;
+    bool count;
+    int group;
+    const uint32_t* rec;
+    int hint;
+    const uint32_t* gids;
+    const uint8_t* window;
+};
+cudaError_t launch_refine_exact(const ExactItems& I, const DArr& A, const DLat& L, const ExactAttr& X,
+                                const ExactOut& out, int sms, cudaStream_t s);
+cudaError_t launch_refine_exact_slab(const ExactItems& I, const DArr& A, const DLat& L, const ExactAttr& X,
+                                     const ExactOut& out, int sms, cudaStream_t s);
+// f64 refinement by a block per entry with `region` bytes of shared memory:
+// work items (list[q], or every item when list is null) or, marked, single
+// edges.  n_dev: the entries' count on the device, at most n_max (null:
+// n_max).  ovf (room for n_max + 1 words): the entries whose lists do not
+// fit, after their count.  rec, hint, gids, window: as launch_refine_exact
+// (rec is needed).
+constexpr size_t BLOCK_HALF_SM = size_t(111) << 10;  // two blocks of this much shared memory to an SM
+struct ExactBlock {
+    const int4* keys;
+    const uint32_t *work, *edges;
+    const float2* edge_vals;
+    const uint32_t *item_off, *item_edges;  // work items
+    const uint32_t* edge_off;               // marked edges
+    uint32_t n_bricks;
+    bool marked;
+    const uint32_t *list, *n_dev;
+    uint32_t n_max;
+    bool wide;  // work items with long lists: 512 threads a block
+    size_t region;
+    uint32_t* ovf;
+    unsigned long long* queue;
+    const uint32_t* rec;
+    int hint;
+    const uint32_t* gids;
+    const uint8_t* window;
+};
+cudaError_t launch_refine_exact_block(const ExactBlock& B, const DArr& A, const DLat& L, const ExactAttr& X,
+                                      const ExactOut& out, int sms, cudaStream_t s);
 void launch_selftest(const float* a, const float* b, uint32_t* out, uint32_t n, cudaStream_t s);
 void launch_scan(const uint32_t* in, uint32_t n, uint32_t* out, uint32_t* keep, unsigned long long* tiles,
                  unsigned long long* total, cudaStream_t s);

@@ -1148,17 +1148,37 @@ int smb_resident_set_exact(smb_resident* r, const uint32_t* orig, const uint32_t
     return SMB_OK;
 }
 
-// The exact refinement of the last run's crossing edges (mask: only the
-// edges k with mask[k] != 0; their results into the vertex buffers).
-static int exact_pass(smb_resident* r, smb_batch* b, const uint8_t* mask, char* err, size_t errlen,
-                      bool count = false) {
+// Shared memory of a block of the exact refinement for lists of up to
+// max_pack units of the gather (their f64 forms take about 2.2 times the
+// bytes): four, two or one block to an SM.
+static size_t exact_block_region(const smb_batch* b, size_t optin) {
+    const size_t need = size_t(b->max_pack) * 36 + 1024;
+    for (size_t r : {size_t(55) << 10, BLOCK_HALF_SM})
+        if (need <= r) return r;
+    return optin - 1024;
+}
+
+// Bytes of the gather's packed lists per sampled sub-block, on average.
+static double exact_mean_list(const smb_batch* b) {
+    return b->n_work ? double(b->pack_units) * 16.0 / double(b->n_work) : 0.0;
+}
+
+static bool exact_wide(const smb_batch* b, int sms) {
+    return exact_mean_list(b) >= 9000.0 || b->n_work < 4u * uint32_t(sms);
+}
+
+// The exact refinement of the last run's crossing edges; with marked, only
+// the first n_marked edges of that list (mask[k] != 0), whose results go into
+// the vertex buffers.
+static int exact_pass(smb_resident* r, smb_batch* b, const uint8_t* mask, const uint32_t* marked, size_t n_marked,
+                      char* err, size_t errlen, bool count = false) {
     smb_device* d = r->dev;
     cudaStream_t s = d->stream;
     const size_t ne = b->n_edges;
     const uint32_t nw = b->n_work;
     int rc;
-    const size_t slab = exact_slab_bytes(d->info.multiprocessors);
-    if ((rc = b->x_ovf.reserve(size_t(nw) * 4 + 8, err, errlen)) || (rc = b->x_slab.reserve(slab, err, errlen)) ||
+    if ((rc = b->x_ovf.reserve((size_t(nw) + 2) * 4, err, errlen)) ||
+        (rc = b->x_ovf2.reserve((std::max<size_t>(nw, n_marked) + 2) * 4, err, errlen)) ||
         (rc = b->item_counts.reserve(size_t(nw) * 4, err, errlen)) ||
         (rc = b->item_off.reserve(size_t(nw) * 4 + 4, err, errlen)) ||
         (rc = b->item_edges.reserve(ne * 4, err, errlen)) ||
@@ -1167,25 +1187,85 @@ static int exact_pass(smb_resident* r, smb_batch* b, const uint8_t* mask, char* 
     b->x_block_items = 0;
     if (!ne || !nw) return SMB_OK;
     unsigned long long* cnt = b->counters.as<unsigned long long>();
+    ExactOut out{b->x_pos.as<float>(), b->x_nrm.as<float>(), b->x_atom.as<uint32_t>(), b->x_patch.as<uint8_t>(),
+                 b->x_t.as<float>(), b->x_evals.as<uint32_t>()};
+    const uint32_t* gids = b->window_ok ? b->ids.as<uint32_t>() : nullptr;
+    const uint8_t* window = b->window_ok ? b->x_window.as<uint8_t>() : nullptr;
+    const int sms = d->info.multiprocessors;
+    const bool blocks = !count && !b->x_group && b->x_region == 0;
+    ExactBlock B{r->keys + b->first, b->work.as<uint32_t>(), b->edges.as<uint32_t>(), b->edge_vals.as<float2>(),
+                 b->item_off.as<uint32_t>(), b->item_edges.as<uint32_t>(), b->edge_off.as<uint32_t>(), b->n,
+                 false, nullptr, nullptr, nw, false, exact_block_region(b, d->smem_optin), b->x_ovf2.as<uint32_t>(),
+                 cnt + CNT_QUEUE, b->rec.as<uint32_t>(), b->x_hint, gids, window};
+    uint32_t over = 0, over_warp = 0;
+    cudaError_t e;
+    // Waits for the passes so far; over: the entries the last one left.
+    auto wait = [&](const DBuf& list) {
+        if (cudaMemcpyAsync(&over_warp, b->x_ovf.p, 4, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
+            cudaMemcpyAsync(&over, list.p, 4, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
+            cudaStreamSynchronize(s) == cudaSuccess)
+            return int(SMB_OK);
+        set_err(err, errlen, "exact refinement: %s", cudaGetErrorString(cudaGetLastError()));
+        return int(SMB_ERR_CUDA);
+    };
+    if (marked && blocks) {
+        B.marked = true, B.list = marked, B.n_max = uint32_t(n_marked);
+        e = launch_refine_exact_block(B, r->A, r->L, r->xa, out, sms, s);
+        if (e != cudaSuccess) return set_err(err, errlen, "exact refine launch: %s", cudaGetErrorString(e)), SMB_ERR_CUDA;
+        if ((rc = wait(b->x_ovf2))) return rc;
+        if (!over) return SMB_OK;
+        // Lists over a block's shared memory: every marked edge again, by
+        // its sub-block's pass below (the results are the same).
+    }
     CK(cudaMemsetAsync(cnt + CNT_MAXITEM, 0, 8, s));
     launch_item_edges(r->L, b->work.as<uint32_t>(), nw, b->rec.as<uint32_t>(), b->edge_off.as<uint32_t>(),
                       b->edges.as<uint32_t>(), b->item_counts.as<uint32_t>(), b->item_off.as<uint32_t>(),
                       b->item_edges.as<uint32_t>(), b->tiles.as<unsigned long long>(),
                       b->totals.as<unsigned long long>() + 3, cnt, s, nullptr, nullptr, mask, true);
-    ExactOut out{b->x_pos.as<float>(), b->x_nrm.as<float>(), b->x_atom.as<uint32_t>(), b->x_patch.as<uint8_t>(),
-                 b->x_t.as<float>(), b->x_evals.as<uint32_t>()};
-    cudaError_t e = launch_refine_exact(r->A, r->L, r->xa, r->keys + b->first, b->work.as<uint32_t>(),
-                                        b->edges.as<uint32_t>(), b->edge_vals.as<float2>(), b->item_off.as<uint32_t>(),
-                                        b->item_edges.as<uint32_t>(), nw, out, b->x_ovf.as<uint32_t>(),
-                                        b->x_slab.as<unsigned char>(), slab, cnt, d->info.multiprocessors,
-                                        b->x_region, s, count, exact_group(b), b->rec.as<uint32_t>(), b->x_hint,
-                                        b->window_ok ? b->ids.as<uint32_t>() : nullptr,
-                                        b->window_ok ? b->x_window.as<uint8_t>() : nullptr);
+    ExactItems I{r->keys + b->first, b->work.as<uint32_t>(), b->edges.as<uint32_t>(), b->edge_vals.as<float2>(),
+                 b->item_off.as<uint32_t>(), b->item_edges.as<uint32_t>(), nw, b->x_ovf.as<uint32_t>(), nullptr, 0,
+                 cnt, b->x_region ? b->x_region : EXACT_REGION, count, exact_group(b), b->rec.as<uint32_t>(),
+                 b->x_hint, gids, window};
+    if (count) CK(cudaMemsetAsync(cnt + CNT_OPS, 0, 8, s));
+    // Which pass takes the sub-blocks.  A warp each needs the fewest
+    // instructions but leaves every list walk and root search to one lane
+    // (a sub-block takes 0.5 to 2 ms), so it pays only where the chip has
+    // many sub-blocks per warp to overlap; blocks of 4 warps (8 lanes per
+    // edge) below five sub-blocks per byte of the mean list, blocks of 16
+    // warps for lists of 9 KB or more and for fewer than four sub-blocks
+    // per SM.  Refinement in ms, warps with overflow to slabs (as before) /
+    // to blocks / narrow blocks / wide blocks:
+    //      241 sub-blocks, lists  4.7 KB:  2.5 /  1.7 /  0.42 /  0.21
+    //    2,753 sub-blocks, lists  5.3 KB:  2.2 /  1.5 /  0.44 /  0.67
+    //   18,752 sub-blocks, lists  6.5 KB:  4.0 /  3.2 /  2.4  /  3.2
+    //   34,492 sub-blocks, lists  8.2 KB:  7.1 /  6.2 /  5.4  /  6.7
+    //   82,359 sub-blocks, lists  3.8 KB:  4.7 /  4.3 /  6.6  / 14
+    //  398,291 sub-blocks, lists  6.8 KB: 44.0 / 43.1 / 51.2  / 86
+    //    8,483 sub-blocks, lists 13.3 KB:  5.9 /  5.4 /  4.0  /  2.7
+    //  106,539 sub-blocks, lists 13.1 KB: 30.4 / 44.8 / 45.7  / 30.2
+    //   17,786 sub-blocks, lists 37.9 KB: 22.3 /  -   / 53    / 16.7
+    const bool wide = exact_wide(b, sms);
+    const bool all_blocks = blocks && (wide || double(nw) < 5.0 * exact_mean_list(b));
+    if (!all_blocks) {
+        e = launch_refine_exact(I, r->A, r->L, r->xa, out, sms, s);
+        if (e != cudaSuccess) return set_err(err, errlen, "exact refine launch: %s", cudaGetErrorString(e)), SMB_ERR_CUDA;
+    }
+    if (blocks) {
+        B.marked = false, B.wide = wide, B.list = nullptr, B.n_dev = nullptr, B.n_max = nw;
+        if (!all_blocks) B.list = I.ovf + 1, B.n_dev = I.ovf;
+        e = launch_refine_exact_block(B, r->A, r->L, r->xa, out, sms, s);
+        if (e != cudaSuccess) return set_err(err, errlen, "exact refine launch: %s", cudaGetErrorString(e)), SMB_ERR_CUDA;
+        I.ovf = b->x_ovf2.as<uint32_t>();
+    }
+    if ((rc = wait(blocks ? b->x_ovf2 : b->x_ovf))) return rc;
+    b->x_block_items = all_blocks ? nw : over_warp;
+    if (!over) return SMB_OK;
+    I.slab_bytes = exact_slab_bytes(sms);
+    if ((rc = b->x_slab.reserve(I.slab_bytes, err, errlen))) return rc;
+    I.slab = b->x_slab.as<unsigned char>();
+    e = launch_refine_exact_slab(I, r->A, r->L, r->xa, out, sms, s);
     if (e != cudaSuccess) return set_err(err, errlen, "exact refine launch: %s", cudaGetErrorString(e)), SMB_ERR_CUDA;
-    uint32_t n_block = 0;
-    CK(cudaMemcpyAsync(&n_block, b->x_ovf.p, 4, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    b->x_block_items = n_block;
     return SMB_OK;
 }
 
@@ -1214,7 +1294,7 @@ int smb_refine_exact(smb_resident* r, smb_batch* b, double* ms, char* err, size_
     if (ms) *ms = 0;
     cudaEventRecord(b->ev[4], s);
     if (b->n_edges) CK(cudaMemsetAsync(b->x_evals.p, 0, b->n_edges * 4, s));
-    if ((rc = exact_pass(r, b, nullptr, err, errlen))) return rc;
+    if ((rc = exact_pass(r, b, nullptr, nullptr, 0, err, errlen))) return rc;
     cudaEventRecord(b->ev[5], s);
     CK(cudaStreamSynchronize(s));
     float t = 0;
@@ -1230,7 +1310,7 @@ int smb_batch_count_exact_ops(smb_batch* b, unsigned long long* ops, char* err, 
     if (!b->refined_exact || b->x_exact_edges != b->n_edges)
         return set_err(err, errlen, "smb_refine_exact must run first"), SMB_ERR_STATE;
     CK(cudaSetDevice(r->dev->index));
-    int rc = exact_pass(r, b, nullptr, err, errlen, true);
+    int rc = exact_pass(r, b, nullptr, nullptr, 0, err, errlen, true);
     if (rc) return rc;
     CK(cudaMemcpy(ops, b->counters.as<unsigned long long>() + CNT_OPS, 8, cudaMemcpyDeviceToHost));
     return SMB_OK;
@@ -1245,7 +1325,9 @@ int smb_place_fast(smb_resident* r, smb_batch* b, double* ms, char* err, size_t 
     cudaStream_t s = d->stream;
     const size_t ne = b->n_edges;
     int rc;
-    if ((rc = reserve_vertices(b, err, errlen)) || (rc = b->x_mask.reserve(ne, err, errlen))) return rc;
+    if ((rc = reserve_vertices(b, err, errlen)) || (rc = b->x_mask.reserve(ne, err, errlen)) ||
+        (rc = b->x_marked.reserve(ne * 4, err, errlen)))
+        return rc;
     b->refined_exact = false;
     if (ms) *ms = 0;
     cudaEventRecord(b->ev[4], s);
@@ -1255,13 +1337,15 @@ int smb_place_fast(smb_resident* r, smb_batch* b, double* ms, char* err, size_t 
     cudaError_t e = launch_place_fast(r->A, r->L, r->xa, r->keys + b->first, b->n, b->edge_off.as<uint32_t>(),
                                       b->edges.as<uint32_t>(), b->edge_vals.as<float2>(), ne, b->e_t.as<float>(),
                                       b->e_feat.as<uint32_t>(), b->e_q.as<float>(), b->e_evals.as<uint32_t>(), out,
-                                      b->x_mask.as<uint8_t>(), marked, s);
+                                      b->x_mask.as<uint8_t>(), b->x_marked.as<uint32_t>(), marked, s);
     if (e != cudaSuccess) return set_err(err, errlen, "placement launch: %s", cudaGetErrorString(e)), SMB_ERR_CUDA;
     unsigned long long n_marked = 0;
     CK(cudaMemcpyAsync(&n_marked, marked, 8, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     b->x_exact_edges = size_t(n_marked);
-    if (n_marked && (rc = exact_pass(r, b, b->x_mask.as<uint8_t>(), err, errlen))) return rc;
+    if (n_marked && (rc = exact_pass(r, b, b->x_mask.as<uint8_t>(), b->x_marked.as<uint32_t>(), size_t(n_marked), err,
+                                     errlen)))
+        return rc;
     cudaEventRecord(b->ev[5], s);
     CK(cudaStreamSynchronize(s));
     float t = 0;

@@ -100,6 +100,10 @@ struct smb_resident {
 // CTAs fit an SM's 228 KiB with their 1 KiB reserve and static bytes.
 constexpr size_t SAMPLE_REGION = 55 * 1024;
 
+// Shared memory of a warp's lists in the exact refinement: four blocks of
+// four warps to an SM.
+constexpr size_t EXACT_REGION = 13312;
+
 struct smb_batch {
     smb_resident* res = nullptr;
     uint32_t n = 0, n_work = 0, max_pack = 0;
@@ -117,13 +121,15 @@ struct smb_batch {
     smb::DBuf item_counts, item_off, item_edges;  // per sampled sub-block edge lists
     // Vertices refined or placed on the device: position, normal, atom, patch,
     // t, evaluations; overflowed items, summary words, fast-mode exact mask.
-    smb::DBuf x_pos, x_nrm, x_atom, x_patch, x_t, x_evals, x_ovf, x_sum, x_mask, x_slab;
+    smb::DBuf x_pos, x_nrm, x_atom, x_patch, x_t, x_evals, x_ovf, x_ovf2, x_sum, x_mask, x_marked, x_slab;
     smb::DBuf x_window;  // per sub-block: the gather's and the exact ball's tests disagree somewhere
     bool window_ok = false;  // x_window and ids are this batch's last gather's (smb_run)
     bool refined_exact = false;
     size_t x_exact_edges = 0;  // edges the exact refinement took in the last pass
     size_t x_block_items = 0;  // items of the last exact pass refined by a whole block
-    size_t x_region = 13312;  // shared-memory bytes per warp for one sub-block's f64 candidate lists
+    // Shared-memory bytes per warp for one sub-block's f64 candidate lists, with
+    // the global-slab pass next (0: EXACT_REGION, with the block pass next).
+    size_t x_region = 0;
     size_t s_region = 0;  // sampling: shared memory of the first pass's CTAs (0: SAMPLE_REGION)
     smb::DBuf s_list;     // sampling: the sub-blocks left to the second pass
     int x_hint = 1;   // smb_refine_exact: list sizes from the gather's records (0 off, 2 one short)
@@ -138,6 +144,6 @@ struct smb_batch {
     std::vector<smb::DBuf*> bufs() {
         return {&rec, &sampled, &work, &retry_a, &retry_b, &values, &tiles, &totals, &counters,
                 &ids, &pack, &mc_counts, &edge_off, &tri_off, &edges, &edge_vals, &tris, &e_t, &e_feat, &e_q, &e_evals, &e_x, &w_feats, &w_start, &item_counts, &item_off, &item_edges,
-                &x_pos, &x_nrm, &x_atom, &x_patch, &x_t, &x_evals, &x_ovf, &x_sum, &x_mask, &x_slab, &s_list, &x_window};
+                &x_pos, &x_nrm, &x_atom, &x_patch, &x_t, &x_evals, &x_ovf, &x_ovf2, &x_sum, &x_mask, &x_marked, &x_slab, &s_list, &x_window};
     }
 };
