@@ -79,8 +79,9 @@ __global__ void k_scan_tile_sums(unsigned long long* tile_sums, uint32_t n_tiles
 // out[i] = exclusive prefix of in; with keep != null, also writes the
 // indices i with in[i] != 0 to keep[prefix] (order-preserving compaction).
 __global__ void k_scan_apply(const uint32_t* in, uint32_t n, const unsigned long long* tile_sums, uint32_t* out,
-                             uint32_t* keep) {
+                             uint32_t* keep, const unsigned long long* tail) {
     __shared__ unsigned long long sh[SCAN_THREADS / 32];
+    if (tail && blockIdx.x == 0 && threadIdx.x == 0) out[n] = uint32_t(*tail);
     uint64_t base = uint64_t(blockIdx.x) * SCAN_TILE + uint64_t(threadIdx.x) * SCAN_ITEMS;
     uint32_t v[SCAN_ITEMS];
     unsigned long long s = 0;
@@ -98,6 +99,37 @@ __global__ void k_scan_apply(const uint32_t* in, uint32_t n, const unsigned long
             if (keep && v[k]) keep[run] = uint32_t(i);
         }
         run += v[k];
+    }
+}
+
+// The same scan by one block, for inputs of a few tiles (the three passes
+// cost three launches, 8 us, whatever the size).
+constexpr int SCAN_SMALL_THREADS = 1024;
+constexpr uint32_t SCAN_SMALL_MAX = 8 * SCAN_TILE;
+__global__ void __launch_bounds__(SCAN_SMALL_THREADS) k_scan_small(const uint32_t* in, uint32_t n, uint32_t* out,
+                                                                   uint32_t* keep, bool tail,
+                                                                   unsigned long long* total) {
+    __shared__ unsigned long long sh[SCAN_SMALL_THREADS / 32];
+    unsigned long long carry = 0;
+    constexpr uint32_t PER = 4;
+    for (uint32_t b0 = 0; b0 < n; b0 += PER * SCAN_SMALL_THREADS) {
+        const uint32_t base = b0 + threadIdx.x * PER;
+        uint32_t v[PER];
+        unsigned long long s = 0, t;
+        for (uint32_t k = 0; k < PER; k++) v[k] = base + k < n ? in[base + k] : 0u, s += v[k];
+        unsigned long long run = carry + block_exclusive_scan<SCAN_SMALL_THREADS>(s, sh, &t);
+        for (uint32_t k = 0; k < PER; k++) {
+            if (base + k < n) {
+                if (out) out[base + k] = uint32_t(run);
+                if (keep && v[k]) keep[run] = base + k;
+            }
+            run += v[k];
+        }
+        carry += t;
+    }
+    if (threadIdx.x == 0) {
+        *total = carry;
+        if (tail) out[n] = uint32_t(carry);
     }
 }
 
@@ -2230,16 +2262,22 @@ void launch_selftest(const float* a, const float* b, uint32_t* out, uint32_t n, 
 }
 
 void launch_scan(const uint32_t* in, uint32_t n, uint32_t* out, uint32_t* keep, unsigned long long* tiles,
-                 unsigned long long* total, cudaStream_t s) {
+                 unsigned long long* total, cudaStream_t s, bool tail) {
     uint32_t n_tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
     if (n_tiles == 0) {
         cudaMemsetAsync(total, 0, sizeof(unsigned long long), s);
+        if (tail) cudaMemsetAsync(out, 0, 4, s);
+        return;
+    }
+    if (n <= SCAN_SMALL_MAX) {
+        COUNT(1);
+        k_scan_small<<<1, SCAN_SMALL_THREADS, 0, s>>>(in, n, out, keep, tail, total);
         return;
     }
     COUNT(3);
     k_scan_tiles<<<n_tiles, SCAN_THREADS, 0, s>>>(in, n, tiles);
     k_scan_tile_sums<<<1, SCAN_THREADS, 0, s>>>(tiles, n_tiles, total);
-    k_scan_apply<<<n_tiles, SCAN_THREADS, 0, s>>>(in, n, tiles, out, keep);
+    k_scan_apply<<<n_tiles, SCAN_THREADS, 0, s>>>(in, n, tiles, out, keep, tail ? total : nullptr);
 }
 
 uint32_t scan_tiles_needed(uint32_t n) { return (n + SCAN_TILE - 1) / SCAN_TILE + 1; }

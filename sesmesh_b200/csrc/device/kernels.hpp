@@ -221,8 +221,11 @@ struct ExactBlock {
 cudaError_t launch_refine_exact_block(const ExactBlock& B, const DArr& A, const DLat& L, const ExactAttr& X,
                                       const ExactOut& out, int sms, cudaStream_t s);
 void launch_selftest(const float* a, const float* b, uint32_t* out, uint32_t n, cudaStream_t s);
+// Exclusive scan of in[0..n) into out (null: not kept) and its total; keep:
+// the indices of the entries != 0 (each 0 or 1), in order; tail: out[n] gets
+// the total too.
 void launch_scan(const uint32_t* in, uint32_t n, uint32_t* out, uint32_t* keep, unsigned long long* tiles,
-                 unsigned long long* total, cudaStream_t s);
+                 unsigned long long* total, cudaStream_t s, bool tail = false);
 uint32_t scan_tiles_needed(uint32_t n);
 void launch_mark_touched(const DArr& A, const DLat& L, const BrickBox& box, uint32_t* flags, int* err, cudaStream_t s,
                          const Scene* many = nullptr, uint32_t n_total = 0);

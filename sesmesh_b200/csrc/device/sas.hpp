@@ -18,6 +18,7 @@ struct DevArrangement {
     const uint32_t* orig = nullptr;          // input index per sphere
     const uint32_t* circle_ij = nullptr;     // 2 per circle
     const uint32_t* vertex_atoms = nullptr;  // 3 per SAS vertex
+    int kind = 0;  // SMB_KIND_*
     size_t n = 0, n_contained = 0, n_circles = 0, n_vertices = 0, nb_items = 0, cb_items = 0;
     double lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};  // bounding box of the centres
     double extent = 0;
@@ -27,10 +28,10 @@ struct DevArrangement {
 // build_arrangement (host/arrangement.cpp, geom/arrangement.rs:246-770) on
 // the device, with the host build's values bit for bit.  0: built; 1: the
 // device declines (an exposure decision within the device's error bound of
-// its threshold, or a circle with more blockers than a thread keeps): the
+// its threshold, or a circle with more blockers than a warp keeps): the
 // caller builds on the host; 2: an error (*msg).
-int build_arrangement_device(smb_device* d, const double* xyzr, size_t n, double probe, DevArrangement& out,
-                             std::string* msg);
+int build_arrangement_device(smb_device* d, const double* xyzr, size_t n, double probe, int kind,
+                             DevArrangement& out, std::string* msg);
 
 // The host Arrangement of a device-built one (the host build's layout).
 bool arrangement_to_host(const DevArrangement& D, smbh::Arrangement& A);

@@ -582,9 +582,9 @@ static void destroy_resident(smb_resident* r) {
     if (r->gone.exchange(true)) return;
     smb_device* d = r->dev;
     cudaSetDevice(d->index);
-    cudaStreamSynchronize(d->stream);
-    for (void* p : r->owned) mem_free(p);
-    if (r->keys) mem_free(r->keys);
+    cudaDeviceSynchronize();  // once for all buffers
+    for (void* p : r->owned) mem_free_synced(p);
+    if (r->keys) mem_free_synced(r->keys);
     delete r;
     dev_release(d);
 }
@@ -630,8 +630,9 @@ int smb_classify(smb_resident* r, size_t* touched, size_t* surface, char* err, s
         return set_err(err, errlen, "brick grid of %.0f bricks exceeds the dense classification limit", ncell), SMB_ERR_RANGE;
     uint32_t nb = uint32_t(ncell);
     DBuf flags, list, surf, cells, tiles, tot, errbuf;
-    auto cleanup = [&] {
-        flags.release(), list.release(), surf.release(), cells.release(), tiles.release(), tot.release(), errbuf.release();
+    auto cleanup = [&] {  // used on this stream alone
+        cudaStreamSynchronize(s);
+        for (DBuf* b : {&flags, &list, &surf, &cells, &tiles, &tot, &errbuf}) b->release_synced();
     };
     int rc;
     if ((rc = flags.reserve(size_t(nb) * 4, err, errlen)) || (rc = list.reserve(size_t(nb) * 4, err, errlen)) ||
@@ -716,8 +717,8 @@ int smb_batch_new(smb_resident* r, smb_batch** out, char* err, size_t errlen) {
 void smb_batch_free(smb_batch* b) {
     if (!b) return;
     cudaSetDevice(b->res->dev->index);
-    cudaStreamSynchronize(b->res->dev->stream);
-    for (DBuf* p : b->bufs()) p->release();
+    cudaDeviceSynchronize();  // once for all buffers
+    for (DBuf* p : b->bufs()) p->release_synced();
     for (auto& ev : b->ev) cudaEventDestroy(ev);
     smb_resident* r = b->res;
     delete b;
@@ -864,12 +865,11 @@ int smb_run(smb_resident* r, size_t first, size_t count, smb_batch* b, smb_batch
     if (e != cudaSuccess) return set_err(err, errlen, "mc launch: %s", cudaGetErrorString(e)), SMB_ERR_CUDA;
     unsigned long long* tot = b->totals.as<unsigned long long>();
     launch_scan(b->mc_counts.as<uint32_t>(), uint32_t(count), b->edge_off.as<uint32_t>(), nullptr,
-                b->tiles.as<unsigned long long>(), tot + 1, s);
+                b->tiles.as<unsigned long long>(), tot + 1, s, true);
     launch_scan(b->mc_counts.as<uint32_t>() + count, uint32_t(count), b->tri_off.as<uint32_t>(), nullptr,
-                b->tiles.as<unsigned long long>(), tot + 2, s);
+                b->tiles.as<unsigned long long>(), tot + 2, s, true);
     unsigned long long t2[3];
     CK(cudaMemcpyAsync(t2, tot, 24, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
     CK(cudaMemcpyAsync(cnt, b->counters.p, CNT_N * 8, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     if (cnt[CNT_TIMEOUT]) return set_err(err, errlen, "a bounded wait for a bulk copy gave up"), SMB_ERR_TIMEOUT;
@@ -877,9 +877,6 @@ int smb_run(smb_resident* r, size_t first, size_t count, smb_batch* b, smb_batch
     b->n_tris = size_t(t2[2]);
     if (b->n_edges >= (size_t(1) << 32) || b->n_tris >= (size_t(1) << 32))
         return set_err(err, errlen, "batch too large for 32-bit offsets"), SMB_ERR_MEMORY;
-    uint32_t ne32 = uint32_t(b->n_edges), nt32 = uint32_t(b->n_tris);
-    CK(cudaMemcpyAsync(b->edge_off.as<uint32_t>() + count, &ne32, 4, cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(b->tri_off.as<uint32_t>() + count, &nt32, 4, cudaMemcpyHostToDevice, s));
     if ((rc = b->edges.reserve(b->n_edges * 4, err, errlen)) || (rc = b->edge_vals.reserve(b->n_edges * 8, err, errlen)) ||
         (rc = b->tris.reserve(b->n_tris * 12, err, errlen)))
         return rc;
@@ -1100,7 +1097,7 @@ int resident_from_device(smb_device* d, DevArrangement& D, const smb_lattice_ref
     r->bytes = D.bytes;
     D.bytes = 0;
     for (int k = 0; k < 3; k++) r->lo[k] = D.lo[k], r->hi[k] = D.hi[k];
-    set_lattice(r->L, lat, D.A.probe, SMB_KIND_SES);
+    set_lattice(r->L, lat, D.A.probe, D.kind);
     r->xa = ExactAttr{D.orig, D.circle_ij, D.vertex_atoms, 0.0};
     *out = r;
     return SMB_OK;
