@@ -262,34 +262,72 @@ __global__ void k_triangle_area_volume(const float* pos, const uint32_t* tris, c
     ta[p] = a, tv[p] = v;
 }
 
-// Thread per segment: its triangles' area and volume summed in triangle
-// order (one (component, chunk) partial of the host's sums).
-constexpr int SEG_WARPS = 4;     // warps (segments) per block of k_segment_partials
-constexpr uint32_t SEG_STAGE = 256;  // values per array a warp stages at a time
+// A warp per (component, chunk) segment: its triangles' areas and volumes
+// summed in triangle order (one partial of the host's sums, in the host's
+// order of additions).  Bound by the latency of up to 16,384 dependent f64
+// additions, so nothing else may stand in the chain: the next stage is copied
+// to shared memory (cp.async, two buffers) while lane 0 adds the areas and
+// lane 1, in the same instructions, the volumes, 16 values read ahead.
+// 16,384 triangles: 254 us with one lane adding both and the copies in
+// between, 100 us so (11 cycles an addition).
+constexpr int SEG_WARPS = 2;         // warps (segments) per block of k_segment_partials
+constexpr uint32_t SEG_STAGE = 512;  // values per array and buffer
+constexpr uint32_t SEG_AHEAD = 16;
 
-// A warp per (component, chunk) segment: the lanes stage the segment's
-// per-triangle areas and volumes in shared memory, coalesced, and lane 0
-// sums them in triangle order (the host's order of additions).
+__device__ __forceinline__ void copy8_async(double* dst, const double* src) {
+    const uint32_t d = uint32_t(__cvta_generic_to_shared(dst));
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
+}
+
 __global__ void __launch_bounds__(32 * SEG_WARPS) k_segment_partials(const double* ta, const double* tv,
                                                                    const uint32_t* comp, const uint32_t* perm,
                                                                    uint32_t nt, const uint32_t* start, uint32_t n_seg,
                                                                    Partial* out, uint32_t* seg_comp) {
-    __shared__ double sa[SEG_WARPS][SEG_STAGE], sv[SEG_WARPS][SEG_STAGE];
+    __shared__ __align__(16) double st[SEG_WARPS][2][2][SEG_STAGE];  // warp, buffer, area or volume
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t s = blockIdx.x * SEG_WARPS + warp;
     if (s >= n_seg) return;
     const uint32_t p0 = start[s], p1 = s + 1 < n_seg ? start[s + 1] : nt;
-    double a = 0.0, v = 0.0;
-    for (uint32_t base = p0; base < p1; base += SEG_STAGE) {
+    auto stage = [&](uint32_t base, int buf) {
         const uint32_t cnt = min(SEG_STAGE, p1 - base);
-        for (uint32_t u = lane; u < cnt; u += 32) sa[warp][u] = ta[base + u], sv[warp][u] = tv[base + u];
+        for (uint32_t u = lane; u < cnt; u += 32) {
+            copy8_async(&st[warp][buf][0][u], ta + base + u);
+            copy8_async(&st[warp][buf][1][u], tv + base + u);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    double sum = 0.0;  // lane 0: area, lane 1: volume
+    int buf = 0;
+    stage(p0, 0);
+    for (uint32_t base = p0; base < p1; base += SEG_STAGE, buf ^= 1) {
+        const uint32_t cnt = min(SEG_STAGE, p1 - base);
+        if (base + SEG_STAGE < p1) {
+            stage(base + SEG_STAGE, buf ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
         __syncwarp();
-        if (lane == 0)
-            for (uint32_t u = 0; u < cnt; u++) a += sa[warp][u], v += sv[warp][u];
+        if (lane < 2) {
+            const double* x = st[warp][buf][lane];
+            uint32_t u = 0;
+            for (; u + SEG_AHEAD <= cnt; u += SEG_AHEAD) {
+                double v[SEG_AHEAD];
+#pragma unroll
+                for (uint32_t k = 0; k < SEG_AHEAD; k += 2) {
+                    const double2 w = *reinterpret_cast<const double2*>(x + u + k);
+                    v[k] = w.x, v[k + 1] = w.y;
+                }
+#pragma unroll
+                for (uint32_t k = 0; k < SEG_AHEAD; k++) sum += v[k];
+            }
+            for (; u < cnt; u++) sum += x[u];
+        }
         __syncwarp();
     }
+    const double volume = __shfl_sync(0xffffffffu, sum, 1);
     if (lane == 0) {
-        out[s] = Partial{comp[p0], perm[p0] / SUM_CHUNK, (unsigned long long)(p1 - p0), a, v};
+        out[s] = Partial{comp[p0], perm[p0] / SUM_CHUNK, (unsigned long long)(p1 - p0), sum, volume};
         seg_comp[s] = comp[p0];
     }
 }
