@@ -817,6 +817,8 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 
 constexpr uint32_t BULK_CHUNK = 32768;            // bytes per bulk copy
 constexpr int SAMPLE_CHUNK = 512;                 // samples per ownership compaction
+constexpr int SAMPLE_THREADS = 128, SAMPLE_THREADS_MAX = 256;
+constexpr uint32_t SAMPLE_SMS = 148;
 constexpr uint32_t MBAR_SPIN_LIMIT = 1u << 24;     // bounded wait
 
 // list (single structure): blocks whose packed block exceeds limit_units
@@ -828,7 +830,7 @@ constexpr uint32_t MBAR_SPIN_LIMIT = 1u << 24;     // bounded wait
 // that set the sample's least distance, the first of equal ones.  Values are
 // the same with and without it.
 template <bool TMA, bool COUNT, bool MANY, bool LIST = false, bool FEAT = false>
-__global__ void __launch_bounds__(128) k_sample(DLat L0, const int4* keys, const uint32_t* work, uint32_t n_work,
+__global__ void __launch_bounds__(SAMPLE_THREADS_MAX) k_sample(DLat L0, const int4* keys, const uint32_t* work, uint32_t n_work,
                                                 const uint32_t* rec, const uint4* pack, float* values,
                                                 unsigned long long* counters, Scene SC, uint32_t limit_units,
                                                 uint32_t* list, const uint32_t* ids, uint32_t* feats) {
@@ -2355,15 +2357,23 @@ cudaError_t launch_sample(const DLat& L, const int4* keys, const uint32_t* work,
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(first));
     if (e != cudaSuccess) return e;
     if (split && (e = cudaMemsetAsync(list, 0, 4, s)) != cudaSuccess) return e;
+    // 256 threads a CTA (a sub-block's samples at the default brick edge take
+    // one round) where the CTAs' shared memory leaves an SM fewer than 40 of
+    // 64 warps with 128, or the sub-blocks are few: 2.4 M spheres at 1 A, 42
+    // KB lists, 299 -> 192 ms; 58,800 at 0.5 A, up to 30 KB, 9.9 -> 8.3; 43
+    // spheres 0.145 -> 0.089; but 58,800 at 0.25 A, up to 17 KB, 18.6 -> 19.9,
+    // the second round of 128 filling its warps better.
+    const bool wide = first > 21 * 1024 || n <= 24u * SAMPLE_SMS;
+    const int threads = wide ? SAMPLE_THREADS_MAX : SAMPLE_THREADS;
     COUNT(1);
-    kern<<<n, 128, first, s>>>(L, keys, work, n, rec, pack, values, counters, many ? *many : Scene{},
+    kern<<<n, threads, first, s>>>(L, keys, work, n, rec, pack, values, counters, many ? *many : Scene{},
                                uint32_t(first / 16), split ? list : nullptr, ids, feats);
     if (!split) return cudaGetLastError();
     auto rest = feat ? k_sample<true, false, false, true, true> : k_sample<true, false, false, true>;
     if ((e = cudaFuncSetAttribute(rest, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))) != cudaSuccess)
         return e;
     COUNT(1);
-    rest<<<n, 128, smem, s>>>(L, keys, work, n, rec, pack, values, counters, Scene{}, 0, list, ids, feats);
+    rest<<<n, threads, smem, s>>>(L, keys, work, n, rec, pack, values, counters, Scene{}, 0, list, ids, feats);
     return cudaGetLastError();
 }
 
