@@ -439,7 +439,7 @@ __device__ __forceinline__ void gather_item(uint32_t item, const DArr& A0, const
     uint32_t* c_off = c_perm + caps.c;
     uint32_t* v_id = c_off + caps.c + 1;
 
-    const uint32_t j = work[item];
+    const uint32_t j = work[size_t(item) * O.stride];
     const uint32_t brick = j >> 3, sb = j & 7;
     uint32_t* rec = O.rec + size_t(j) * REC_WORDS;
     const int4 key = keys[brick];

@@ -46,6 +46,7 @@ struct GatherOut {
     // exact refinement's ball test (rho with its margins) but not the
     // gather's or the other way round, else 0.
     uint8_t* window = nullptr;
+    uint32_t stride = 1;  // work item i is work[i * stride] (a sample of the items)
 };
 
 // Fast-mode refinement constants (RefineRef, sesmesh-gpu batch.rs:133-150).

@@ -708,7 +708,7 @@ int smb_batch_new(smb_resident* r, smb_batch** out, char* err, size_t errlen) {
         smb_device* d = r->dev;
         std::lock_guard<std::mutex> g(d->hint_mu);
         if (d->hint.warps && d->hint.b == r->L.b && d->hint.h == r->L.h && d->hint.probe == r->A.probe)
-            b->caps = d->hint.caps, b->gather_warps = d->hint.warps;
+            b->caps = d->hint.caps, b->gather_warps = d->hint.warps, b->caps_seen = true;
     }
     *out = b;
     return SMB_OK;
@@ -724,6 +724,11 @@ void smb_batch_free(smb_batch* b) {
     delete b;
     if (r->refs.fetch_sub(1) == 1 && r->freed.load()) destroy_resident(r);
 }
+
+// From this many sampled sub-blocks on, the gather's list pools are sized to
+// what they need.
+static constexpr size_t GATHER_SAMPLE_MIN = 8192;
+static constexpr uint32_t GATHER_SAMPLE_STRIDE = 64;
 
 int smb_run(smb_resident* r, size_t first, size_t count, smb_batch* b, smb_batch_times* times, char* err,
             size_t errlen) {
@@ -773,9 +778,55 @@ int smb_run(smb_resident* r, size_t first, size_t count, smb_batch* b, smb_batch
     // (b) gather, with list memory grown and shared-memory caps raised as
     // needed (bit-identical results at any capacity).
     GatherCaps caps = b->caps;
+    int warps = b->gather_warps;
     unsigned long long cnt[CNT_N];
-    size_t want_ids = std::max<size_t>(b->ids.cap / 4, size_t(n_work) * 1024),
-           want_pack = std::max<size_t>(b->pack.cap / 16, size_t(n_work) * 512);
+    size_t want_ids = b->ids.cap / 4, want_pack = b->pack.cap / 16;
+    double ids_per = 0, units_per = 0;
+    {
+        std::lock_guard<std::mutex> g(d->hint_mu);
+        if (d->hint.b == L.b && d->hint.h == L.h && d->hint.probe == r->A.probe)
+            ids_per = d->hint.ids_per, units_per = d->hint.units_per;
+    }
+    if (n_work < GATHER_SAMPLE_MIN) {
+        // 48 KB a sub-block: at most 400 MB.
+        want_ids = std::max<size_t>(want_ids, size_t(n_work) * 4096);
+        want_pack = std::max<size_t>(want_pack, size_t(n_work) * 2048);
+    } else if (!want_ids || !want_pack) {
+        // The pools' sizes from an earlier structure's lists with these
+        // lattice and probe values, else from every 64th sub-block gathered
+        // without pools (nothing is written; 0.16 ms and 1.5 % of the gather):
+        // a pass that runs past its pools is run again, which costs all of it
+        // (2.4 M spheres at 1 A, 42 KB a sub-block in pools of 13: 476 ms,
+        // with the right ones 259).
+        if (!ids_per) {
+            const uint32_t some = uint32_t((n_work + GATHER_SAMPLE_STRIDE - 1) / GATHER_SAMPLE_STRIDE);
+            CK(cudaMemsetAsync(b->counters.p, 0, CNT_N * 8, s));
+            GatherOut O{b->rec.as<uint32_t>(), nullptr, nullptr, b->retry_a.as<uint32_t>(),
+                        b->counters.as<unsigned long long>(), 0, 0, ~0ull, nullptr, nullptr, GATHER_SAMPLE_STRIDE};
+            cudaError_t e = launch_gather(r->A, L, keys, b->work.as<uint32_t>(), some, O, caps, warps, s);
+            if (e != cudaSuccess)
+                return set_err(err, errlen, "gather launch: %s", cudaGetErrorString(e)), SMB_ERR_CUDA;
+            CK(cudaMemcpyAsync(cnt, b->counters.p, CNT_N * 8, cudaMemcpyDeviceToHost, s));
+            CK(cudaStreamSynchronize(s));
+            // A sub-block over the caps counts as four of the others.
+            const double over = double(cnt[CNT_OVERFLOW]), counted = std::max(double(some) - over, 1.0);
+            ids_per = double(cnt[CNT_IDS]) / double(some) * (1.0 + 4.0 * over / counted);
+            units_per = double(cnt[CNT_PACK]) / double(some) * (1.0 + 4.0 * over / counted);
+            // No earlier caps either: the sample's largest lists and a quarter
+            // (sub-blocks over them are gathered again with larger ones).
+            if (!b->caps_seen && !cnt[CNT_OVERFLOW]) {
+                auto up = [](unsigned long long v) { return std::max(32, int((v + v / 4 + 16 + 15) / 16 * 16)); };
+                GatherCaps seen{up(cnt[CNT_MAXNN]), up(cnt[CNT_MAXNS]), up(cnt[CNT_MAXNC]), up(cnt[CNT_MAXNV])};
+                const size_t per = gather_smem_bytes(seen);
+                if (per <= gather_smem_bytes(caps)) {
+                    caps = seen;
+                    warps = int(std::max<size_t>(1, std::min<size_t>(8, size_t(65536) / per)));
+                }
+            }
+        }
+        want_ids = std::max<size_t>(size_t(ids_per * 1.25 * double(n_work)), size_t(n_work) * 256);
+        want_pack = std::max<size_t>(size_t(units_per * 1.25 * double(n_work)), size_t(n_work) * 128);
+    }
     for (int attempt = 0;; attempt++) {
         if ((rc = b->ids.reserve(want_ids * 4, err, errlen)) || (rc = b->pack.reserve(want_pack * 16, err, errlen)))
             return rc;
@@ -783,7 +834,7 @@ int smb_run(smb_resident* r, size_t first, size_t count, smb_batch* b, smb_batch
         GatherOut O{b->rec.as<uint32_t>(), b->ids.as<uint32_t>(), b->pack.as<uint4>(), b->retry_a.as<uint32_t>(),
                     b->counters.as<unsigned long long>(), b->ids.cap / 4, b->pack.cap / 16, ~0ull, nullptr,
                     b->x_window.as<uint8_t>()};
-        cudaError_t e = launch_gather(r->A, L, keys, b->work.as<uint32_t>(), uint32_t(n_work), O, caps, b->gather_warps, s);
+        cudaError_t e = launch_gather(r->A, L, keys, b->work.as<uint32_t>(), uint32_t(n_work), O, caps, warps, s);
         if (e != cudaSuccess) return set_err(err, errlen, "gather launch: %s", cudaGetErrorString(e)), SMB_ERR_CUDA;
         CK(cudaMemcpyAsync(cnt, b->counters.p, CNT_N * 8, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
@@ -835,10 +886,15 @@ int smb_run(smb_resident* r, size_t first, size_t count, smb_batch* b, smb_batch
         size_t per = gather_smem_bytes(next);
         if (per <= size_t(d->smem_optin)) {
             b->caps = next;
+            b->caps_seen = true;
             b->gather_warps = int(std::max<size_t>(1, std::min<size_t>(8, size_t(65536) / per)));
             std::lock_guard<std::mutex> g(d->hint_mu);
-            d->hint.h = L.h, d->hint.b = L.b, d->hint.probe = r->A.probe;
-            d->hint.caps = b->caps, d->hint.warps = b->gather_warps;
+            smb_device::CapsHint& H = d->hint;
+            if (H.h != L.h || H.b != L.b || H.probe != r->A.probe) H.ids_per = H.units_per = 0;
+            H.h = L.h, H.b = L.b, H.probe = r->A.probe;
+            H.caps = b->caps, H.warps = b->gather_warps;
+            if (n_work >= GATHER_SAMPLE_MIN)
+                H.ids_per = double(cnt[CNT_IDS]) / double(n_work), H.units_per = double(cnt[CNT_PACK]) / double(n_work);
         }
     }
     cudaEventRecord(b->ev[2], s);

@@ -72,6 +72,7 @@ struct smb_device {
         int b = 0;
         smb::GatherCaps caps{};
         int warps = 0;
+        double ids_per = 0, units_per = 0;  // list words and units per sub-block, runs of many sub-blocks (0: none yet)
     } hint;
 };
 
@@ -139,6 +140,7 @@ struct smb_batch {
     size_t r_region = 0;  // smb_refine: bytes per warp's f32 region when four whole ones do not fit (0: an eighth of the SM's)
     smb::GatherCaps caps{192, 128, 384, 128};
     int gather_warps = 4;
+    bool caps_seen = false;  // caps are those of an earlier run with these lattice and probe values
     bool use_tma = true;
     cudaEvent_t ev[6] = {};
     std::vector<smb::DBuf*> bufs() {
