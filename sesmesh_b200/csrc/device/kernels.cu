@@ -2111,6 +2111,7 @@ constexpr int REFINE_WARPS = 4;
 // refinement (ten or more blocks to an SM; at most 80 registers, so twelve
 // blocks where the regions allow).
 constexpr size_t PAIR_REGION_MAX = 20480;
+constexpr size_t MANY_REGION = 14 * 1024;  // and of the many-structure pass's
 
 struct RefinePlan {
     uint32_t cand_bytes;  // one staging region
@@ -2352,7 +2353,7 @@ cudaError_t launch_sample(const DLat& L, const int4* keys, const uint32_t* work,
     // Shared memory for the largest block on every CTA can leave an SM a
     // few CTAs: the blocks up to `small` bytes run first with that much,
     // the rest after them with all of it.
-    const bool split = list && !many && !count && tma && small >= 16 && smem > small;
+    const bool split = list && !count && tma && small >= 16 && smem > small;
     const size_t first = split ? small / 16 * 16 : smem;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(first));
     if (e != cudaSuccess) return e;
@@ -2369,11 +2370,13 @@ cudaError_t launch_sample(const DLat& L, const int4* keys, const uint32_t* work,
     kern<<<n, threads, first, s>>>(L, keys, work, n, rec, pack, values, counters, many ? *many : Scene{},
                                uint32_t(first / 16), split ? list : nullptr, ids, feats);
     if (!split) return cudaGetLastError();
-    auto rest = feat ? k_sample<true, false, false, true, true> : k_sample<true, false, false, true>;
+    auto rest = feat ? (many ? k_sample<true, false, true, true, true> : k_sample<true, false, false, true, true>)
+                     : (many ? k_sample<true, false, true, true> : k_sample<true, false, false, true>);
     if ((e = cudaFuncSetAttribute(rest, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))) != cudaSuccess)
         return e;
     COUNT(1);
-    rest<<<n, threads, smem, s>>>(L, keys, work, n, rec, pack, values, counters, Scene{}, 0, list, ids, feats);
+    rest<<<n, threads, smem, s>>>(L, keys, work, n, rec, pack, values, counters, many ? *many : Scene{}, 0, list, ids,
+                                  feats);
     return cudaGetLastError();
 }
 
@@ -2448,17 +2451,16 @@ cudaError_t launch_refine(const DArr& A, const DLat& L, const RefineConsts& RC, 
     P.cand_bytes = uint32_t(al(cand_bytes));
     const size_t narrow = size_t(REFINE_WARPS) * P.cand_bytes;
     const size_t wide = P.cand_bytes;
-    // One staging region per warp (an item per warp in flight, as many items
-    // per SM as regions fit) while four fit in a block, else one per block.
-    // The single-structure pass instead gives blocks of two warps one region
-    // each: of the largest sub-block's size where that is at most
-    // PAIR_REGION_MAX, else of the size asked for (default: an eighth of the
-    // SM's shared memory), handing the sub-blocks that outgrow it to a
-    // whole-block pass over a list.
+    // Blocks of two warps that share one staging region per sub-block: of the
+    // largest sub-block's size where that is at most PAIR_REGION_MAX, else of
+    // the size asked for (default: an eighth of the SM's shared memory),
+    // handing the sub-blocks that outgrow it to a whole-block pass over a
+    // list.  The counting pass (and a caller without ovf): one region per
+    // warp while four fit in a block, else one per block.
     const bool use_wide = narrow > smem_limit;
     size_t small = region ? region / 128 * 128 : (smem_limit / 2 - 1024) / REFINE_WARPS / 128 * 128;
     small = std::max<size_t>(std::min(small, size_t(P.cand_bytes)), 128);
-    const bool split = !many && ovf && (use_wide || small < P.cand_bytes);
+    const bool split = ovf && (use_wide || small < P.cand_bytes);
     const size_t smem = use_wide ? wide : narrow;
     if (smem_out) *smem_out = smem;
     if (!n_items) return cudaSuccess;
@@ -2502,6 +2504,26 @@ cudaError_t launch_refine(const DArr& A, const DLat& L, const RefineConsts& RC, 
         auto kp = warm ? k_refine<REFINE_WARM, true, false, 8, 64> : k_refine<REFINE_PLAIN, true, false, 8, 64>;
         return run(kp, P, wide, nullptr, nullptr, n_items, 64);
     }
+    if (many) {
+        // Many structures: the largest block of any of them sets cand_bytes,
+        // so most sub-blocks take a small region (14 KB: 180.5 ms for the
+        // device stages of 64 structures, 187 at 20 KB, 197 at 28).  A lane
+        // per edge and one block of four warps to an SM, which the largest
+        // lists left, took 19.4 ms for ten structures of 20 to 5,000 spheres
+        // at 0.1 to 0.5 A; this takes 7.1.
+        if (!ovf) return cudaErrorInvalidValue;
+        RefinePlan PS = P;
+        PS.cand_bytes = uint32_t(std::min<size_t>(small, MANY_REGION));
+        cudaError_t e = cudaMemsetAsync(ovf, 0, 4, s);
+        if (e != cudaSuccess) return e;
+        auto kp = warm ? k_refine<REFINE_WARM, true, true, 8, 64, false, true>
+                       : k_refine<REFINE_PLAIN, true, true, 8, 64, false, true>;
+        if ((e = run(kp, PS, PS.cand_bytes, ovf, nullptr, n_items, 64)) != cudaSuccess) return e;
+        if (PS.cand_bytes >= P.cand_bytes) return cudaSuccess;
+        auto kw = warm ? k_refine<REFINE_WARM, true, true, 32, 32 * WIDE_LIST_WARPS>
+                       : k_refine<REFINE_PLAIN, true, true, 32, 32 * WIDE_LIST_WARPS>;
+        return run(kw, P, wide, nullptr, ovf, n_items, 32 * WIDE_LIST_WARPS);
+    }
     if (split) {
         RefinePlan PS = P;
         PS.cand_bytes = uint32_t(small);
@@ -2522,15 +2544,10 @@ cudaError_t launch_refine(const DArr& A, const DLat& L, const RefineConsts& RC, 
         if (e != cudaSuccess) return e;
         return run(kw, P, wide, nullptr, ovf, n_items, 32 * WIDE_LIST_WARPS);
     }
-    // Groups of lanes per edge: one lane in the many-structure pass (short
-    // lists, few evaluations after the warm start), else 8 or 32 as asked.
-    auto kern =
-        many ? (warm ? pick(k_refine<REFINE_WARM, false, true, 1>, k_refine<REFINE_WARM, true, true, 1>)
-                     : pick(k_refine<REFINE_PLAIN, false, true, 1>, k_refine<REFINE_PLAIN, true, true, 1>))
-        : warm ? (g32 ? pick(k_refine<REFINE_WARM, false, false, 32>, k_refine<REFINE_WARM, true, false, 32>)
-                      : pick(k_refine<REFINE_WARM, false, false, 8>, k_refine<REFINE_WARM, true, false, 8>))
-               : (g32 ? pick(k_refine<REFINE_PLAIN, false, false, 32>, k_refine<REFINE_PLAIN, true, false, 32>)
-                      : pick(k_refine<REFINE_PLAIN, false, false, 8>, k_refine<REFINE_PLAIN, true, false, 8>));
+    auto kern = warm ? (g32 ? pick(k_refine<REFINE_WARM, false, false, 32>, k_refine<REFINE_WARM, true, false, 32>)
+                            : pick(k_refine<REFINE_WARM, false, false, 8>, k_refine<REFINE_WARM, true, false, 8>))
+                     : (g32 ? pick(k_refine<REFINE_PLAIN, false, false, 32>, k_refine<REFINE_PLAIN, true, false, 32>)
+                            : pick(k_refine<REFINE_PLAIN, false, false, 8>, k_refine<REFINE_PLAIN, true, false, 8>));
     return run(kern, P, smem, nullptr, nullptr, use_wide ? n_items : quads);
 }
 

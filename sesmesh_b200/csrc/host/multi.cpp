@@ -62,6 +62,11 @@ struct CapLevel {
     uint32_t unit_cap;
     uint32_t ids_per_sub, units_per_sub;
 };
+// Shared memory of the first sampling pass's CTAs: one pass holds structures
+// of every spacing, so the largest lists say little about most (64 structures
+// at brick edge 8, 229 ms at 55 KB, 215 at 20 KB or less; at edge 16, 187 and
+// 181).
+constexpr size_t MANY_SAMPLE_REGION = 20 * 1024;
 const CapLevel CAP_LEVELS[2] = {
     {{192, 128, 384, 128}, 2048, 640, 320},
     {{384, 256, 768, 256}, 8192, 1280, 640},
@@ -136,6 +141,7 @@ struct smb_multi {
     DBuf flags, list, surf, cells, tiles, tot, keys, rec, sampled, work, retry, values, counters, totals, ids, pack;
     DBuf mc_counts, edge_off, tri_off, edges, edge_vals, tris, item_counts, item_off, item_edges;
     DBuf e_t, e_feat, e_q, e_evals;
+    DBuf s_list, r_ovf;     // sub-blocks left to the sampling's and the refinement's second passes
     DBuf w_feats, w_start;  // warm start: the sampler's nearest features, each row's start
     size_t edge_cap = 0, tri_cap = 0;
     // Groups of structures, one pass (and one recorded graph) each.
@@ -160,7 +166,7 @@ struct smb_multi {
         return {&d_arr, &d_lat, &d_rc, &d_box, &d_flag_off, &d_sph_off, &d_err, &d_fail, &flags, &list, &surf,
                 &cells, &tiles, &tot, &keys, &rec, &sampled, &work, &retry, &values, &counters, &totals, &ids, &pack,
                 &mc_counts, &edge_off, &tri_off, &edges, &edge_vals, &tris, &item_counts, &item_off, &item_edges, &w_feats, &w_start,
-                &e_t, &e_feat, &e_q, &e_evals};
+                &e_t, &e_feat, &e_q, &e_evals, &s_list, &r_ovf};
     }
     size_t n() const { return eng.size(); }
 };
@@ -326,6 +332,7 @@ int reserve_pass(smb_multi* m, size_t max_nb, char* err, size_t errlen) {
     int rc;
     if ((rc = m->rec.reserve(nsub * REC_WORDS * 4, err, errlen)) || (rc = m->sampled.reserve(nsub * 4, err, errlen)) ||
         (rc = m->work.reserve(nsub * 4, err, errlen)) || (rc = m->retry.reserve(nsub * 4, err, errlen)) ||
+        (rc = m->s_list.reserve(nsub * 4 + 4, err, errlen)) || (rc = m->r_ovf.reserve(nsub * 4 + 4, err, errlen)) ||
         (rc = m->values.reserve(nb * spb * 4, err, errlen)) ||
         (rc = m->tiles.reserve(size_t(scan_tiles_needed(uint32_t(nsub))) * 8 + 64, err, errlen)) ||
         (rc = m->counters.reserve(CNT_N * 8, err, errlen)) ||
@@ -345,12 +352,10 @@ int reserve_pass(smb_multi* m, size_t max_nb, char* err, size_t errlen) {
     return SMB_OK;
 }
 
-// The mesh-stage pass over one group's surface bricks (keys [k0, k1)), all
-// sizes fixed (no host synchronisation inside), as one stream of launches:
-// recorded once into a CUDA graph, then replayed.
-int enqueue_pass(smb_multi* m, const Group& G, char* err, size_t errlen) {
+// The first part of a group's pass (keys [k0, k1)): sub-block states and the
+// candidate lists.
+int enqueue_lists(smb_multi* m, const Group& G, char* err, size_t errlen) {
     cudaStream_t s = m->dev->stream;
-    smb_device* d = m->dev;
     const uint32_t nb = uint32_t(G.k1 - G.k0), nsub = nb * 8;
     const int b = m->cfg.brick;
     const CapLevel& C = CAP_LEVELS[m->cfg.caps_level];
@@ -359,8 +364,6 @@ int enqueue_pass(smb_multi* m, const Group& G, char* err, size_t errlen) {
     const int4* keys = m->keys.as<int4>() + G.k0;
     unsigned long long* cnt = m->counters.as<unsigned long long>();
     unsigned long long* tot = m->totals.as<unsigned long long>();
-    DLat L{};  // per-structure lattices come from the scene; b and spb are shared
-    L.b = b, L.sub = b / 2, L.spb = int(spb);
     MCK(cudaMemsetAsync(cnt, 0, CNT_N * 8, s));
     MCK(cudaMemsetAsync(m->values.p, 0, size_t(nb) * spb * 4, s));
     launch_substates(DArr{}, DLat{}, keys, nb, m->rec.as<uint32_t>(), m->sampled.as<uint32_t>(), s, &S);
@@ -385,9 +388,26 @@ int enqueue_pass(smb_multi* m, const Group& G, char* err, size_t errlen) {
         e = launch_gather(DArr{}, DLat{}, keys, m->retry.as<uint32_t>(), nsub, O2, big, 1, s, &R);
         if (e != cudaSuccess) return set_err(err, errlen, "gather launch: %s", cudaGetErrorString(e)), SMB_ERR_CUDA;
     }
-    e = launch_sample(DLat{}, keys, m->work.as<uint32_t>(), nsub, m->rec.as<uint32_t>(), m->pack.as<uint4>(),
-                      m->unit_cap, m->values.as<float>(), cnt, true, false, s, &S, nullptr, 0, m->ids.as<uint32_t>(),
-                      m->warm ? m->w_feats.as<uint32_t>() : nullptr);
+    return SMB_OK;
+}
+
+// The rest of it: sampling, marching cubes, refinement.
+int enqueue_mesh(smb_multi* m, const Group& G, char* err, size_t errlen) {
+    cudaStream_t s = m->dev->stream;
+    smb_device* d = m->dev;
+    const uint32_t nb = uint32_t(G.k1 - G.k0), nsub = nb * 8;
+    const int b = m->cfg.brick;
+    const size_t spb = size_t(b + 1) * (b + 1) * (b + 1);
+    Scene S = scene_of(m);
+    const int4* keys = m->keys.as<int4>() + G.k0;
+    unsigned long long* cnt = m->counters.as<unsigned long long>();
+    unsigned long long* tot = m->totals.as<unsigned long long>();
+    DLat L{};  // per-structure lattices come from the scene; b and spb are shared
+    L.b = b, L.sub = b / 2, L.spb = int(spb);
+    cudaError_t e = launch_sample(DLat{}, keys, m->work.as<uint32_t>(), nsub, m->rec.as<uint32_t>(),
+                                  m->pack.as<uint4>(), m->unit_cap, m->values.as<float>(), cnt, true, false, s, &S,
+                                  m->s_list.as<uint32_t>(), MANY_SAMPLE_REGION, m->ids.as<uint32_t>(),
+                                  m->warm ? m->w_feats.as<uint32_t>() : nullptr);
     if (e != cudaSuccess) return set_err(err, errlen, "sample launch: %s", cudaGetErrorString(e)), SMB_ERR_CUDA;
     e = launch_mc(L, nb, m->values.as<float>(), m->rec.as<uint32_t>(), m->mc_counts.as<uint32_t>(), nullptr, nullptr,
                   nullptr, nullptr, nullptr, false, s, keys, ~0ull, ~0ull, &S);
@@ -420,9 +440,16 @@ int enqueue_pass(smb_multi* m, const Group& G, char* err, size_t errlen) {
                       m->item_off.as<uint32_t>(), m->item_edges.as<uint32_t>(), nsub, m->e_t.as<float>(),
                       m->e_feat.as<uint32_t>(), m->e_q.as<float>(), m->e_evals.as<uint32_t>(), cand, mode,
                       m->warm ? m->w_start.as<float2>() : nullptr, cnt, d->info.multiprocessors, d->smem_optin, s,
-                      nullptr, &S);
+                      nullptr, &S, m->r_ovf.as<uint32_t>());
     if (e != cudaSuccess) return set_err(err, errlen, "refine launch: %s", cudaGetErrorString(e)), SMB_ERR_CUDA;
     return SMB_OK;
+}
+
+// The whole pass, all sizes fixed (no host synchronisation inside), as one
+// stream of launches: recorded once into a CUDA graph, then replayed.
+int enqueue_pass(smb_multi* m, const Group& G, char* err, size_t errlen) {
+    int rc = enqueue_lists(m, G, err, errlen);
+    return rc ? rc : enqueue_mesh(m, G, err, errlen);
 }
 
 // Runs one group's pass: from its recorded graph when that matches the
@@ -439,16 +466,16 @@ int run_group(smb_multi* m, Group& G, float* device_ms, char* err, size_t errlen
                       G.gen == m->gen;
     if (!same) {
         if (G.graph) cudaGraphExecDestroy(G.graph), G.graph = nullptr;
-        // Direct passes: the first sets the kernels' attributes; when lists
-        // ran past the pools or the sampler's block cap, those grow to what
-        // the pass counted and the pass runs again (twice at most).
+        // A direct pass (which sets the kernels' attributes).  When its lists
+        // run past the pools or the sampler's block cap, those grow to what
+        // it counted and the lists are gathered again (twice at most) before
+        // anything is built on them.
+        MCK(cudaEventRecord(m->ev[0], s));
         for (int attempt = 0;; attempt++) {
-            MCK(cudaEventRecord(m->ev[0], s));
-            if ((rc = enqueue_pass(m, G, err, errlen))) return rc;
-            MCK(cudaEventRecord(m->ev[1], s));
-            MCK(cudaStreamSynchronize(s));
+            if ((rc = enqueue_lists(m, G, err, errlen))) return rc;
             unsigned long long c[CNT_N];
-            MCK(cudaMemcpy(c, m->counters.p, sizeof c, cudaMemcpyDeviceToHost));
+            MCK(cudaMemcpyAsync(c, m->counters.p, sizeof c, cudaMemcpyDeviceToHost, s));
+            MCK(cudaStreamSynchronize(s));
             if (!c[CNT_NOMEM] || attempt >= 2) break;
             bool grow = false;
             if (c[CNT_IDS] > m->ids.cap / 4) {
@@ -468,6 +495,9 @@ int run_group(smb_multi* m, Group& G, float* device_ms, char* err, size_t errlen
             m->gen++;
             MCK(cudaMemsetAsync(m->d_fail.as<uint32_t>() + G.s0, 0, (G.s1 - G.s0) * 4, s));
         }
+        if ((rc = enqueue_mesh(m, G, err, errlen))) return rc;
+        MCK(cudaEventRecord(m->ev[1], s));
+        MCK(cudaStreamSynchronize(s));
         cudaGraph_t g = nullptr;
         if (m->graph_ok && cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
             char e2[256] = {0};
@@ -763,6 +793,7 @@ int finish_structure_device(smb_multi* m, const Group& G, size_t i, const uint32
     b->window_ok = false;  // the slice brings records, not the gather's ids or marks
     b->n = uint32_t(nb);
     b->n_work = uint32_t(nw);
+    b->max_pack = m->unit_cap;  // at most
     b->n_edges = ne;
     b->n_tris = nt;
     b->refined = true;
