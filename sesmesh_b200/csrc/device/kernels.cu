@@ -206,10 +206,10 @@ __device__ __forceinline__ void cell_key(const BrickBox& box, uint32_t cell, int
 // each touched brick's centre, one warp per brick.
 template <bool MANY>
 __global__ void k_classify_bricks(DArr A0, DLat L0, BrickBox box0, const uint32_t* touched, uint32_t n_touched,
-                                  uint32_t* surface, Scene S) {
+                                  const unsigned long long* n_dev, uint32_t* surface, Scene S) {
     uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int lane = threadIdx.x & 31;
-    if (w >= n_touched) return;
+    if (w >= (n_dev ? uint32_t(*n_dev) : n_touched)) return;
     const uint32_t flag = touched[w];
     uint32_t st = 0, cell = flag;
     if constexpr (MANY) {
@@ -228,9 +228,10 @@ __global__ void k_classify_bricks(DArr A0, DLat L0, BrickBox box0, const uint32_
 }
 
 template <bool MANY>
-__global__ void k_cells_to_keys(BrickBox box0, const uint32_t* cells, uint32_t n, int4* keys, Scene S) {
+__global__ void k_cells_to_keys(BrickBox box0, const uint32_t* cells, uint32_t n, const unsigned long long* n_dev,
+                                int4* keys, Scene S) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    if (i >= (n_dev ? uint32_t(*n_dev) : n)) return;
     uint32_t st = 0, cell = cells[i];
     if constexpr (MANY) {
         st = structure_of(S.flag_off, S.n_struct, (unsigned long long)cell);
@@ -774,7 +775,7 @@ template <bool MANY, bool WIDE>
 __global__ void __launch_bounds__(256, MANY ? 2 : 4) k_gather(DArr A0, DLat L0, const int4* keys, const uint32_t* work, uint32_t n_work, GatherOut O,
                          GatherCaps caps, Scene S) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const uint32_t n = MANY ? uint32_t(*S.n_work) : n_work;
+    const uint32_t n = S.n_work ? uint32_t(*S.n_work) : n_work;
     const uint32_t wpb = blockDim.x >> 5;
     for (uint32_t item = blockIdx.x * wpb + (threadIdx.x >> 5); item < n; item += gridDim.x * wpb)
         gather_item<MANY, WIDE>(item, A0, L0, keys, work, O, caps, S, smem_raw);
@@ -829,8 +830,8 @@ constexpr uint32_t MBAR_SPIN_LIMIT = 1u << 24;     // bounded wait
 // 3 circle, 4 SAS vertex; ids of the structure's arrangement): the candidate
 // that set the sample's least distance, the first of equal ones.  Values are
 // the same with and without it.
-template <bool TMA, bool COUNT, bool MANY, bool LIST = false, bool FEAT = false>
-__global__ void __launch_bounds__(SAMPLE_THREADS_MAX) k_sample(DLat L0, const int4* keys, const uint32_t* work, uint32_t n_work,
+template <bool TMA, bool COUNT, bool MANY, bool LIST = false, bool FEAT = false, int NT = SAMPLE_THREADS>
+__global__ void __launch_bounds__(NT) k_sample(DLat L0, const int4* keys, const uint32_t* work, uint32_t n_work,
                                                 const uint32_t* rec, const uint4* pack, float* values,
                                                 unsigned long long* counters, Scene SC, uint32_t limit_units,
                                                 uint32_t* list, const uint32_t* ids, uint32_t* feats) {
@@ -2296,19 +2297,23 @@ void launch_mark_touched(const DArr& A, const DLat& L, const BrickBox& box, uint
 }
 
 void launch_classify_bricks(const DArr& A, const DLat& L, const BrickBox& box, const uint32_t* touched, uint32_t n,
-                            uint32_t* surface, cudaStream_t s, const Scene* many) {
+                            uint32_t* surface, cudaStream_t s, const Scene* many, const unsigned long long* n_dev) {
     if (!n) return;
     COUNT(1);
-    if (many) k_classify_bricks<true><<<(n + 7) / 8, 256, 0, s>>>(A, L, box, touched, n, surface, *many);
-    else k_classify_bricks<false><<<(n + 7) / 8, 256, 0, s>>>(A, L, box, touched, n, surface, Scene{});
+    // Few bricks: a warp a block, so that they spread over the SMs.
+    const uint32_t warps = n <= 148 * 16 ? 1 : 8;
+    if (many) k_classify_bricks<true><<<(n + 7) / 8, 256, 0, s>>>(A, L, box, touched, n, n_dev, surface, *many);
+    else
+        k_classify_bricks<false><<<(n + warps - 1) / warps, 32 * warps, 0, s>>>(A, L, box, touched, n, n_dev, surface,
+                                                                               Scene{});
 }
 
 void launch_cells_to_keys(const BrickBox& box, const uint32_t* cells, uint32_t n, int4* keys, cudaStream_t s,
-                          const Scene* many) {
+                          const Scene* many, const unsigned long long* n_dev) {
     if (!n) return;
     COUNT(1);
-    if (many) k_cells_to_keys<true><<<(n + 255) / 256, 256, 0, s>>>(box, cells, n, keys, *many);
-    else k_cells_to_keys<false><<<(n + 255) / 256, 256, 0, s>>>(box, cells, n, keys, Scene{});
+    if (many) k_cells_to_keys<true><<<(n + 255) / 256, 256, 0, s>>>(box, cells, n, n_dev, keys, *many);
+    else k_cells_to_keys<false><<<(n + 255) / 256, 256, 0, s>>>(box, cells, n, n_dev, keys, Scene{});
 }
 
 void launch_substates(const DArr& A, const DLat& L, const int4* keys, uint32_t n, uint32_t* rec, uint32_t* sampled,
@@ -2320,7 +2325,8 @@ void launch_substates(const DArr& A, const DLat& L, const int4* keys, uint32_t n
 }
 
 cudaError_t launch_gather(const DArr& A, const DLat& L, const int4* keys, const uint32_t* work, uint32_t n,
-                          const GatherOut& O, const GatherCaps& caps, int warps, cudaStream_t s, const Scene* many) {
+                          const GatherOut& O, const GatherCaps& caps, int warps, cudaStream_t s, const Scene* many,
+                          const unsigned long long* n_dev) {
     if (!n) return cudaSuccess;
     size_t smem = gather_smem_bytes(caps) * size_t(warps);
     // Lists of several warp rounds (the caps come from the largest lists
@@ -2333,7 +2339,10 @@ cudaError_t launch_gather(const DArr& A, const DLat& L, const int4* keys, const 
     // strides (a few waves of blocks, not one per possible item).
     uint32_t blocks = (n + warps - 1) / warps;
     if (many) blocks = std::min<uint32_t>(blocks, 148u * 32u);
-    kern<<<blocks, 32 * warps, smem, s>>>(A, L, keys, work, n, O, caps, many ? *many : Scene{});
+    Scene S{};
+    if (many) S = *many;
+    else S.n_work = n_dev;
+    kern<<<blocks, 32 * warps, smem, s>>>(A, L, keys, work, n, O, caps, S);
     return cudaGetLastError();
 }
 
@@ -2344,20 +2353,11 @@ cudaError_t launch_sample(const DLat& L, const int4* keys, const uint32_t* work,
     if (!n) return cudaSuccess;
     size_t smem = size_t(max_units) * 16;
     const bool feat = feats != nullptr && !count;
-    auto kern = feat ? (many ? k_sample<true, false, true, false, true>
-                             : (tma ? k_sample<true, false, false, false, true>
-                                    : k_sample<false, false, false, false, true>))
-                     : many ? k_sample<true, false, true>
-                     : (count ? k_sample<true, true, false>
-                              : (tma ? k_sample<true, false, false> : k_sample<false, false, false>));
     // Shared memory for the largest block on every CTA can leave an SM a
     // few CTAs: the blocks up to `small` bytes run first with that much,
     // the rest after them with all of it.
     const bool split = list && !count && tma && small >= 16 && smem > small;
     const size_t first = split ? small / 16 * 16 : smem;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(first));
-    if (e != cudaSuccess) return e;
-    if (split && (e = cudaMemsetAsync(list, 0, 4, s)) != cudaSuccess) return e;
     // 256 threads a CTA (a sub-block's samples at the default brick edge take
     // one round) where the CTAs' shared memory leaves an SM fewer than 40 of
     // 64 warps with 128, or the sub-blocks are few: 2.4 M spheres at 1 A, 42
@@ -2365,19 +2365,35 @@ cudaError_t launch_sample(const DLat& L, const int4* keys, const uint32_t* work,
     // spheres 0.145 -> 0.089; but 58,800 at 0.25 A, up to 17 KB, 18.6 -> 19.9,
     // the second round of 128 filling its warps better.
     const bool wide = first > 21 * 1024 || n <= 24u * SAMPLE_SMS;
-    const int threads = wide ? SAMPLE_THREADS_MAX : SAMPLE_THREADS;
-    COUNT(1);
-    kern<<<n, threads, first, s>>>(L, keys, work, n, rec, pack, values, counters, many ? *many : Scene{},
-                               uint32_t(first / 16), split ? list : nullptr, ids, feats);
-    if (!split) return cudaGetLastError();
-    auto rest = feat ? (many ? k_sample<true, false, true, true, true> : k_sample<true, false, false, true, true>)
-                     : (many ? k_sample<true, false, true, true> : k_sample<true, false, false, true>);
-    if ((e = cudaFuncSetAttribute(rest, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))) != cudaSuccess)
-        return e;
-    COUNT(1);
-    rest<<<n, threads, smem, s>>>(L, keys, work, n, rec, pack, values, counters, many ? *many : Scene{}, 0, list, ids,
-                                  feats);
-    return cudaGetLastError();
+    auto go = [&](auto nt) -> cudaError_t {
+        constexpr int NT = decltype(nt)::value;
+        auto kern = feat ? (many ? k_sample<true, false, true, false, true, NT>
+                                 : (tma ? k_sample<true, false, false, false, true, NT>
+                                        : k_sample<false, false, false, false, true, NT>))
+                         : many ? k_sample<true, false, true, false, false, NT>
+                                : (count ? k_sample<true, true, false, false, false, NT>
+                                         : (tma ? k_sample<true, false, false, false, false, NT>
+                                                : k_sample<false, false, false, false, false, NT>));
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(first));
+        if (e != cudaSuccess) return e;
+        if (split && (e = cudaMemsetAsync(list, 0, 4, s)) != cudaSuccess) return e;
+        COUNT(1);
+        kern<<<n, NT, first, s>>>(L, keys, work, n, rec, pack, values, counters, many ? *many : Scene{},
+                                  uint32_t(first / 16), split ? list : nullptr, ids, feats);
+        if (!split) return cudaGetLastError();
+        auto rest = feat ? (many ? k_sample<true, false, true, true, true, NT>
+                                 : k_sample<true, false, false, true, true, NT>)
+                         : (many ? k_sample<true, false, true, true, false, NT>
+                                 : k_sample<true, false, false, true, false, NT>);
+        if ((e = cudaFuncSetAttribute(rest, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))) != cudaSuccess)
+            return e;
+        COUNT(1);
+        rest<<<n, NT, smem, s>>>(L, keys, work, n, rec, pack, values, counters, many ? *many : Scene{}, 0, list, ids,
+                                 feats);
+        return cudaGetLastError();
+    };
+    return wide ? go(std::integral_constant<int, SAMPLE_THREADS_MAX>{})
+                : go(std::integral_constant<int, SAMPLE_THREADS>{});
 }
 
 cudaError_t launch_mc(const DLat& L, uint32_t n, float* values, const uint32_t* rec, uint32_t* counts, const uint32_t* edge_off,

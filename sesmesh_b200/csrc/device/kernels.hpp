@@ -230,15 +230,18 @@ void launch_scan(const uint32_t* in, uint32_t n, uint32_t* out, uint32_t* keep, 
 uint32_t scan_tiles_needed(uint32_t n);
 void launch_mark_touched(const DArr& A, const DLat& L, const BrickBox& box, uint32_t* flags, int* err, cudaStream_t s,
                          const Scene* many = nullptr, uint32_t n_total = 0);
+// n_dev: the count of touched bricks (cells, gathered sub-blocks) on the
+// device, at most n (null: n).
 void launch_classify_bricks(const DArr& A, const DLat& L, const BrickBox& box, const uint32_t* touched, uint32_t n,
-                            uint32_t* surface, cudaStream_t s, const Scene* many = nullptr);
+                            uint32_t* surface, cudaStream_t s, const Scene* many = nullptr,
+                            const unsigned long long* n_dev = nullptr);
 void launch_cells_to_keys(const BrickBox& box, const uint32_t* cells, uint32_t n, int4* keys, cudaStream_t s,
-                          const Scene* many = nullptr);
+                          const Scene* many = nullptr, const unsigned long long* n_dev = nullptr);
 void launch_substates(const DArr& A, const DLat& L, const int4* keys, uint32_t n, uint32_t* rec, uint32_t* sampled,
                       cudaStream_t s, const Scene* many = nullptr);
 cudaError_t launch_gather(const DArr& A, const DLat& L, const int4* keys, const uint32_t* work, uint32_t n,
                           const GatherOut& O, const GatherCaps& caps, int warps, cudaStream_t s,
-                          const Scene* many = nullptr);
+                          const Scene* many = nullptr, const unsigned long long* n_dev = nullptr);
 // One CTA per sampled sub-block with the largest packed block's bytes of
 // shared memory; with list (n + 1 words) and small, two passes: the blocks
 // of up to small bytes with small bytes each, then the others.

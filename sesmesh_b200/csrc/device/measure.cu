@@ -281,13 +281,16 @@ __device__ __forceinline__ void copy8_async(double* dst, const double* src) {
 
 __global__ void __launch_bounds__(32 * SEG_WARPS) k_segment_partials(const double* ta, const double* tv,
                                                                    const uint32_t* comp, const uint32_t* perm,
-                                                                   uint32_t nt, const uint32_t* start, uint32_t n_seg,
+                                                                   uint32_t nt, const uint32_t* start,
+                                                                   const unsigned long long* n_segments, uint32_t cap,
                                                                    Partial* out, uint32_t* seg_comp) {
+    const unsigned long long n_all = *n_segments;
+    const uint32_t n_seg = uint32_t(min(n_all, (unsigned long long)cap));
     __shared__ __align__(16) double st[SEG_WARPS][2][2][SEG_STAGE];  // warp, buffer, area or volume
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t s = blockIdx.x * SEG_WARPS + warp;
     if (s >= n_seg) return;
-    const uint32_t p0 = start[s], p1 = s + 1 < n_seg ? start[s + 1] : nt;
+    const uint32_t p0 = start[s], p1 = s + 1 < n_all ? start[s + 1] : nt;
     auto stage = [&](uint32_t base, int buf) {
         const uint32_t cnt = min(SEG_STAGE, p1 - base);
         for (uint32_t u = lane; u < cnt; u += 32) {
@@ -332,24 +335,24 @@ __global__ void __launch_bounds__(32 * SEG_WARPS) k_segment_partials(const doubl
     }
 }
 
-// Partials in (component, chunk) order (sorted_idx: their order, or null
-// for the identity): each component sums its chunks in chunk order (the
-// host's order).
-__global__ void k_component_sums(const Partial* parts, const uint32_t* sorted_idx, uint32_t n_parts,
-                                 const uint32_t* first, uint32_t n_comp, unsigned long long* tris_out, double* area,
-                                 double* volume) {
+// Partials in (component, chunk) order: each component sums its chunks in
+// chunk order (the host's order).
+__global__ void k_component_sums(const Partial* parts, const uint32_t* first, uint32_t n_comp,
+                                 unsigned long long* tris_out, double* area, double* volume) {
     uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= n_comp) return;
     unsigned long long t = 0;
     double a = 0.0, v = 0.0;
     for (uint32_t i = first[c]; i < first[c + 1]; i++) {
-        const Partial& p = parts[sorted_idx ? sorted_idx[i] : i];
+        const Partial& p = parts[i];
         t += p.t, a += p.a, v += p.v;
     }
     tris_out[c] = t, area[c] = a, volume[c] = v;
 }
 
-__global__ void k_first_of_component(const uint32_t* sorted_comp, uint32_t n, uint32_t* first, uint32_t n_comp) {
+__global__ void k_first_of_component(const uint32_t* sorted_comp, const unsigned long long* n_segments, uint32_t cap,
+                                     uint32_t* first, uint32_t n_comp) {
+    const uint32_t n = uint32_t(min(*n_segments, (unsigned long long)cap));
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i > n) return;
     // first[c] = the first sorted index with component >= c.
@@ -468,8 +471,7 @@ unsigned bits_for(uint32_t n) {
 
 void MeasureScratch::release(bool synced) {
     for (DBuf* b : {&pos, &nrm, &tris, &tris_out, &keys, &cnt, &dup, &parent, &flag, &cid, &id, &counters, &comp_v,
-                    &comp_t, &area, &volume, &parts, &pkey, &pidx, &pkey2, &pidx2, &first, &tkey, &tidx,
-                    &tkey2, &tidx2, &tiles, &cub, &packed, &err, &tri_a, &tri_v})
+                    &parts, &pkey, &first, &tkey, &tidx, &tkey2, &tidx2, &tiles, &cub, &packed, &tri_a, &tri_v})
         synced ? b->release_synced() : b->release();
     pinned_free(host);
     host = nullptr;
@@ -487,9 +489,14 @@ __global__ void k_read_words(const unsigned long long* src, unsigned long long* 
 // nrm may be null; tris: 3 u32 per triangle).  Results: comps, *bad, and,
 // when there are no defects, each vertex's component into host_comp and the
 // regrouped triangles into host_tris (nv and 3 nt words on the host).
+// assembled: the triangles come from k_assemble on this stream (indices in
+// range) with S.counters cleared before it; its error word (counter 6) goes
+// to *assembled, and nothing more is done when it is set.  The device is
+// waited for twice (three times otherwise): once for the checks and the
+// components' number, once for the results.
 static bool measure_core(smb_device* d, const float* pos, const float* nrm, const uint32_t* tris, size_t nv,
                          size_t nt, std::vector<smbh::Component>& comps, size_t* bad, MeasureScratch& S,
-                         std::string* msg, uint32_t* host_comp, uint32_t* host_tris) {
+                         std::string* msg, uint32_t* host_comp, uint32_t* host_tris, unsigned long long* assembled) {
     using smbh::Component;
     cudaStream_t s = d->stream;
     if (nv >= (size_t(1) << 31) || nt >= (size_t(1) << 31)) {
@@ -507,8 +514,9 @@ static bool measure_core(smb_device* d, const float* pos, const float* nrm, cons
         if (msg) *msg = std::string("device memory for the measure: ") + e;
         return false;
     }
-    unsigned long long* cnt = S.counters.as<unsigned long long>();  // 0 bad, 1 oob, 2 parts, 3 overflow, 4 comps, 5 union-find
-    MCK(cudaMemsetAsync(cnt, 0, 64, s));
+    // 0 bad, 1 oob, 2 parts, 3 overflow, 4 comps, 5 union-find, 6 assembly
+    unsigned long long* cnt = S.counters.as<unsigned long long>();
+    if (!assembled) MCK(cudaMemsetAsync(cnt, 0, 64, s));
     if (!S.words && !(S.words = static_cast<unsigned long long*>(pinned_alloc(64)))) {
         if (msg) *msg = "page-locked counter words";
         return false;
@@ -522,16 +530,19 @@ static bool measure_core(smb_device* d, const float* pos, const float* nrm, cons
     };
     auto blocks = [](uint64_t n) { return unsigned((n + 255) / 256); };
     if (nv) k_vertex_checks<<<blocks(nv), 256, 0, s>>>(pos, nrm, uint32_t(nv), cnt);
-    if (nt) k_index_checks<<<blocks(nt), 256, 0, s>>>(tris, uint32_t(nt), uint32_t(nv), cnt + 1);
-    if (!pull()) {
-        if (msg) *msg = "measure checks";
-        return false;
+    if (nt && !assembled) {
+        k_index_checks<<<blocks(nt), 256, 0, s>>>(tris, uint32_t(nt), uint32_t(nv), cnt + 1);
+        if (!pull()) {
+            if (msg) *msg = "measure checks";
+            return false;
+        }
+        if (W[1]) {  // indices out of range: the host counts one defect more and stops there
+            *bad = size_t(W[0] + 1);
+            return true;
+        }
     }
-    if (W[1]) {  // indices out of range: the host counts one defect more and stops there
-        *bad = size_t(W[0] + 1);
-        return true;
-    }
-    if (nt) {
+    uint32_t* parent = S.parent.as<uint32_t>();
+    if (nt && nv) {
         k_triangle_checks<<<blocks(nt), 256, 0, s>>>(pos, tris, uint32_t(nt), cnt);
         MCK(cudaMemsetAsync(S.keys.p, 0xFF, ecap * 8, s));
         MCK(cudaMemsetAsync(S.cnt.p, 0, ecap * 8, s));
@@ -542,15 +553,7 @@ static bool measure_core(smb_device* d, const float* pos, const float* nrm, cons
                                                   cnt);
         k_duplicates<<<blocks(nt), 256, 0, s>>>(tris, uint32_t(nt), S.dup.as<uint32_t>(), dcap - 1, cnt);
     }
-    if (!pull()) {
-        if (msg) *msg = "measure checks";
-        return false;
-    }
-    const unsigned long long nbad = W[0];
-    *bad = size_t(nbad);
-    if (nbad) return true;
     // Components.
-    uint32_t* parent = S.parent.as<uint32_t>();
     if (nv) {
         k_uf_init<<<blocks(nv), 256, 0, s>>>(parent, uint32_t(nv));
         if (nt) k_uf_link<<<blocks(nt), 256, 0, s>>>(tris, uint32_t(nt), parent, cnt + 5);
@@ -559,24 +562,29 @@ static bool measure_core(smb_device* d, const float* pos, const float* nrm, cons
                     S.tiles.as<unsigned long long>(), cnt + 4, s);
     }
     if (!pull()) {
-        if (msg) *msg = "measure components";
+        if (msg) *msg = "measure checks";
         return false;
     }
-    const unsigned long long n_comp = W[4], uf_fail = W[5];
-    if (uf_fail) {
+    if (assembled && (*assembled = W[6])) return true;
+    *bad = size_t(W[0]);
+    if (*bad) return true;
+    if (W[5]) {
         if (msg) *msg = "union-find gave up";
         return false;
     }
-    const uint32_t nc = uint32_t(n_comp);
-    if (!R(S.comp_v, size_t(nc) * 8) || !R(S.comp_t, size_t(nc) * 8) ||
-        !R(S.area, size_t(nc) * 8) || !R(S.volume, size_t(nc) * 8) || !R(S.first, (size_t(nc) + 1) * 4)) {
+    const uint32_t nc = uint32_t(W[4]);
+    // Per component: vertices, triangles, area, volume.
+    if (!R(S.comp_v, size_t(nc) * 32 + 8) || !R(S.first, (size_t(nc) + 1) * 4)) {
         if (msg) *msg = std::string("device memory for the measure: ") + e;
         return false;
     }
-    MCK(cudaMemsetAsync(S.comp_v.p, 0, size_t(nc) * 8 + 8, s));
+    unsigned long long* comp_v = S.comp_v.as<unsigned long long>();
+    unsigned long long* comp_t = comp_v + nc;
+    double* comp_a = reinterpret_cast<double*>(comp_t + nc);
+    double* comp_vol = comp_a + nc;
+    MCK(cudaMemsetAsync(comp_v, 0, size_t(nc) * 32 + 8, s));
     uint32_t* id = S.id.as<uint32_t>();
-    if (nv) k_component_ids<<<blocks(nv), 256, 0, s>>>(parent, S.cid.as<uint32_t>(), uint32_t(nv), id,
-                                                       S.comp_v.as<unsigned long long>());
+    if (nv) k_component_ids<<<blocks(nv), 256, 0, s>>>(parent, S.cid.as<uint32_t>(), uint32_t(nv), id, comp_v);
     // Arrays that are final go back on the copy stream while the main one
     // computes the rest; the end of this function waits for both.
     cudaStream_t cs = d->copy ? d->copy : s;
@@ -632,53 +640,58 @@ static bool measure_core(smb_device* d, const float* pos, const float* nrm, cons
     // Area and volume: one partial per (component, 16,384-triangle chunk)
     // summed in triangle order, then each component's partials in chunk
     // order (the host's operations in the host's order).  The sorted
-    // triangles list the segments in (component, chunk) order.
-    unsigned long long n_seg = 0;
+    // triangles list the segments in (component, chunk) order.  Room for four
+    // segments per component and chunk is nearly always enough (their number
+    // stays on the device); a mesh with more sums again with what it needs.
+    const uint64_t chunks = (uint64_t(nt) + SUM_CHUNK - 1) / SUM_CHUNK;
+    uint32_t cap = uint32_t(std::min<uint64_t>(std::max<uint64_t>(nt, 1), 4 * (nc + chunks) + 256));
     if (nt) {
+        if (!R(S.tri_a, nt * 8) || !R(S.tri_v, nt * 8)) {
+            if (msg) *msg = std::string("device memory for the measure: ") + e;
+            return false;
+        }
         uint32_t* flag = S.tkey.as<uint32_t>();   // free once sorted
         uint32_t* start = S.tidx.as<uint32_t>();  // idem
         k_segment_flags<<<blocks(nt), 256, 0, s>>>(S.tkey2.as<uint32_t>(), S.tidx2.as<uint32_t>(), uint32_t(nt), flag);
         launch_scan(flag, uint32_t(nt), nullptr, start, S.tiles.as<unsigned long long>(), cnt + 2, s);
-        if (!pull()) {
-            if (msg) *msg = "measure segments";
-            return false;
-        }
-        n_seg = W[2];
-    }
-    const uint32_t np = uint32_t(n_seg);
-    if (np) {
-        if (!R(S.parts, size_t(np) * sizeof(Partial)) || !R(S.pkey, size_t(np) * 4) || !R(S.tri_a, nt * 8) ||
-            !R(S.tri_v, nt * 8)) {
-            if (msg) *msg = std::string("device memory for the measure: ") + e;
-            return false;
-        }
-        Partial* parts = S.parts.as<Partial>();
         k_triangle_area_volume<<<blocks(nt), 256, 0, s>>>(pos, tris, S.tidx2.as<uint32_t>(), uint32_t(nt),
                                                           S.tri_a.as<double>(), S.tri_v.as<double>());
-        k_segment_partials<<<(np + SEG_WARPS - 1) / SEG_WARPS, 32 * SEG_WARPS, 0, s>>>(
-            S.tri_a.as<double>(), S.tri_v.as<double>(),
-                                                      S.tkey2.as<uint32_t>(), S.tidx2.as<uint32_t>(), uint32_t(nt),
-                                                      S.tidx.as<uint32_t>(), np, parts, S.pkey.as<uint32_t>());
-        k_first_of_component<<<blocks(uint64_t(np) + 1), 256, 0, s>>>(S.pkey.as<uint32_t>(), np,
-                                                                        S.first.as<uint32_t>(), nc);
-        k_component_sums<<<blocks(nc), 256, 0, s>>>(parts, nullptr, np, S.first.as<uint32_t>(), nc,
-                                                    S.comp_t.as<unsigned long long>(), S.area.as<double>(),
-                                                    S.volume.as<double>());
-    } else if (nc) {
-        MCK(cudaMemsetAsync(S.comp_t.p, 0, size_t(nc) * 8, s));
-        MCK(cudaMemsetAsync(S.area.p, 0, size_t(nc) * 8, s));
-        MCK(cudaMemsetAsync(S.volume.p, 0, size_t(nc) * 8, s));
     }
-    // Results to the host.
-    std::vector<unsigned long long> cv(nc), ct(nc);
-    std::vector<double> ca(nc), cvol(nc);
-    if (nc) {
-        MCK(cudaMemcpyAsync(cv.data(), S.comp_v.p, size_t(nc) * 8, cudaMemcpyDeviceToHost, s));
-        MCK(cudaMemcpyAsync(ct.data(), S.comp_t.p, size_t(nc) * 8, cudaMemcpyDeviceToHost, s));
-        MCK(cudaMemcpyAsync(ca.data(), S.area.p, size_t(nc) * 8, cudaMemcpyDeviceToHost, s));
-        MCK(cudaMemcpyAsync(cvol.data(), S.volume.p, size_t(nc) * 8, cudaMemcpyDeviceToHost, s));
+    struct Pinned {
+        void* p;
+        ~Pinned() { pinned_free(p); }
+    } res{pinned_alloc(size_t(nc) * 32 + 8)};
+    if (!res.p) {
+        if (msg) *msg = "page-locked results";
+        return false;
     }
-    MCK(cudaStreamSynchronize(s));
+    for (;;) {
+        if (nt) {
+            if (!R(S.parts, size_t(cap) * sizeof(Partial)) || !R(S.pkey, size_t(cap) * 4)) {
+                if (msg) *msg = std::string("device memory for the measure: ") + e;
+                return false;
+            }
+            Partial* parts = S.parts.as<Partial>();
+            k_segment_partials<<<(cap + SEG_WARPS - 1) / SEG_WARPS, 32 * SEG_WARPS, 0, s>>>(
+                S.tri_a.as<double>(), S.tri_v.as<double>(), S.tkey2.as<uint32_t>(), S.tidx2.as<uint32_t>(),
+                uint32_t(nt), S.tidx.as<uint32_t>(), cnt + 2, cap, parts, S.pkey.as<uint32_t>());
+            k_first_of_component<<<blocks(uint64_t(cap) + 1), 256, 0, s>>>(S.pkey.as<uint32_t>(), cnt + 2, cap,
+                                                                             S.first.as<uint32_t>(), nc);
+            k_component_sums<<<blocks(nc), 256, 0, s>>>(parts, S.first.as<uint32_t>(), nc, comp_t, comp_a, comp_vol);
+        }
+        // Results to the host.
+        MCK(cudaMemcpyAsync(res.p, comp_v, size_t(nc) * 32 + 8, cudaMemcpyDeviceToHost, s));
+        if (!pull()) {
+            if (msg) *msg = "measure results";
+            return false;
+        }
+        if (!nt || W[2] <= cap) break;
+        cap = uint32_t(W[2]);
+    }
+    const unsigned long long* cv = static_cast<const unsigned long long*>(res.p);
+    const unsigned long long* ct = cv + nc;
+    const double* ca = reinterpret_cast<const double*>(ct + nc);
+    const double* cvol = ca + nc;
     comps.assign(nc, Component());
     size_t start = 0;
     for (uint32_t c = 0; c < nc; c++) {
@@ -713,7 +726,8 @@ bool measure_on_device(smb_device* d, smbh::Mesh& m, std::vector<smbh::Component
     MCK(cudaMemcpyAsync(S.tris.p, m.triangles.data(), nt * 12, cudaMemcpyHostToDevice, s));
     m.vertex_component.resize(nv);
     return measure_core(d, S.pos.as<float>(), normals ? S.nrm.as<float>() : nullptr, S.tris.as<uint32_t>(), nv, nt,
-                        comps, bad, S, msg, m.vertex_component.data(), reinterpret_cast<uint32_t*>(m.triangles.data()));
+                        comps, bad, S, msg, m.vertex_component.data(), reinterpret_cast<uint32_t*>(m.triangles.data()),
+                        nullptr);
 }
 
 void* MeasureScratch::staging(size_t bytes) {
@@ -738,7 +752,7 @@ int finish_on_device(smb_device* d, const DeviceMesh& in, smbh::MeshRef* out, vo
     }
     char e[256];
     auto R = [&](DBuf& b, size_t bytes) { return b.reserve(std::max<size_t>(bytes, 16), e, sizeof e) == 0; };
-    if (!R(S.packed, size_t(in.n_bricks) * 8) || !R(S.tris, nt * 12) || !R(S.err, 16)) {
+    if (!R(S.packed, size_t(in.n_bricks) * 8) || !R(S.tris, nt * 12) || !R(S.counters, 64)) {
         if (msg) *msg = std::string("device memory for the assembly: ") + e;
         return 1;
     }
@@ -748,31 +762,6 @@ int finish_on_device(smb_device* d, const DeviceMesh& in, smbh::MeshRef* out, vo
         if (msg) *msg = "page-locked staging memory";
         return 1;
     }
-    auto t0 = std::chrono::steady_clock::now();
-    auto blocks = [](uint64_t n) { return unsigned((n + 255) / 256); };
-    unsigned long long* err = S.err.as<unsigned long long>();
-    if (cudaMemsetAsync(err, 0, 8, s) != cudaSuccess) return 1;
-    k_packed_keys<<<blocks(in.n_bricks), 256, 0, s>>>(in.keys, uint32_t(in.n_bricks), S.packed.as<unsigned long long>(),
-                                                      err);
-    if (nt)
-        k_assemble<<<blocks(nt), 256, 0, s>>>(S.packed.as<unsigned long long>(), in.keys, uint32_t(in.n_bricks),
-                                              in.edge_off, in.edges, in.tri_off, in.tri_refs, uint32_t(nt),
-                                              S.tris.as<uint32_t>(), err);
-    count_launches(nt ? 2 : 1);
-    unsigned long long ferr = 0;
-    if (cudaMemcpyAsync(&ferr, err, 8, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaStreamSynchronize(s) != cudaSuccess) {
-        if (msg) *msg = "device assembly failed";
-        return 1;
-    }
-    if (ms_assemble) *ms_assemble = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-    if (ferr) {
-        if (msg)
-            *msg = (ferr & 4) ? "bricks are not in packed-key order"
-                   : (ferr & 1) ? "triangle references an edge of a missing brick"
-                                : "triangle references an edge without vertex";
-        return 2;
-    }
     // Staging layout: positions, normals (12 B each), atoms, components
     // (4 B), patches (1 B) per vertex, then the triangles.
     unsigned char* h_pos = H;
@@ -781,9 +770,10 @@ int finish_on_device(smb_device* d, const DeviceMesh& in, smbh::MeshRef* out, vo
     unsigned char* h_comp = h_atom + nv * 4;
     unsigned char* h_patch = h_comp + nv * 4;
     unsigned char* h_tris = h_patch + nv;
-    // The vertex arrays go back on the copy stream while the measure's
-    // kernels run on the main one (the copies wait for everything the main
-    // stream has queued so far); every return below waits for them.
+    // The vertex arrays go back on the copy stream while the assembly's and
+    // the measure's kernels run on the main one (the copies wait for
+    // everything the main stream has queued so far); every return below
+    // waits for them.
     cudaStream_t cs = d->copy ? d->copy : s;
     struct Join {
         cudaStream_t c;
@@ -804,6 +794,18 @@ int finish_on_device(smb_device* d, const DeviceMesh& in, smbh::MeshRef* out, vo
             return 1;
         }
     }
+    auto t0 = std::chrono::steady_clock::now();
+    auto blocks = [](uint64_t n) { return unsigned((n + 255) / 256); };
+    unsigned long long* err = S.counters.as<unsigned long long>() + 6;
+    if (cudaMemsetAsync(S.counters.p, 0, 64, s) != cudaSuccess) return 1;
+    k_packed_keys<<<blocks(in.n_bricks), 256, 0, s>>>(in.keys, uint32_t(in.n_bricks), S.packed.as<unsigned long long>(),
+                                                      err);
+    if (nt)
+        k_assemble<<<blocks(nt), 256, 0, s>>>(S.packed.as<unsigned long long>(), in.keys, uint32_t(in.n_bricks),
+                                              in.edge_off, in.edges, in.tri_off, in.tri_refs, uint32_t(nt),
+                                              S.tris.as<uint32_t>(), err);
+    count_launches(nt ? 2 : 1);
+    if (ms_assemble) *ms_assemble = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     auto d2h = [&](void* dst, const void* src, size_t bytes) {
         return !bytes || cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, cs) == cudaSuccess;
     };
@@ -812,9 +814,18 @@ int finish_on_device(smb_device* d, const DeviceMesh& in, smbh::MeshRef* out, vo
         if (msg) *msg = "vertex copy";
         return 1;
     }
+    // The assembly's corners are all below nv (0 where it reports an error).
+    unsigned long long ferr = 0;
     if (!measure_core(d, in.pos, in.nrm, S.tris.as<uint32_t>(), nv, nt, comps, bad, S, msg,
-                      reinterpret_cast<uint32_t*>(h_comp), reinterpret_cast<uint32_t*>(h_tris)))
+                      reinterpret_cast<uint32_t*>(h_comp), reinterpret_cast<uint32_t*>(h_tris), &ferr))
         return 1;
+    if (ferr) {
+        if (msg)
+            *msg = (ferr & 4) ? "bricks are not in packed-key order"
+                   : (ferr & 1) ? "triangle references an edge of a missing brick"
+                                : "triangle references an edge without vertex";
+        return 2;
+    }
     if (*bad) return 0;
     // The staging block becomes the mesh's storage.
     out->pos = reinterpret_cast<const float*>(h_pos);

@@ -11,9 +11,8 @@ namespace smb {
 
 // Device buffers of the measure, kept between meshes.
 struct MeasureScratch {
-    DBuf pos, nrm, tris, tris_out, keys, cnt, dup, parent, flag, cid, id, counters, comp_v, comp_t, area,
-        volume, parts, pkey, pidx, pkey2, pidx2, first, tkey, tidx, tkey2, tidx2, tiles, cub, packed, err, tri_a,
-        tri_v;
+    DBuf pos, nrm, tris, tris_out, keys, cnt, dup, parent, flag, cid, id, counters, comp_v, parts, pkey, first, tkey,
+        tidx, tkey2, tidx2, tiles, cub, packed, tri_a, tri_v;
     void* host = nullptr;  // page-locked staging of the results
     size_t host_cap = 0;
     // Page-locked words the device writes counters into directly: reading

@@ -168,9 +168,8 @@ uint64_t smb_engine_device_bytes(const smb_engine* e) {
         for (smb::DBuf* b : const_cast<smb_batch*>(e->batch)->bufs()) n += b->cap;
     smb::MeasureScratch& M = const_cast<smb_engine*>(e)->measure;
     for (smb::DBuf* b : {&M.pos, &M.nrm, &M.tris, &M.tris_out, &M.keys, &M.cnt, &M.dup, &M.parent, &M.flag, &M.cid,
-                         &M.id, &M.counters, &M.comp_v, &M.comp_t, &M.area, &M.volume, &M.parts, &M.pkey, &M.pidx,
-                         &M.pkey2, &M.pidx2, &M.first, &M.tkey, &M.tidx, &M.tkey2, &M.tidx2, &M.tiles, &M.cub,
-                         &M.packed, &M.err, &M.tri_a, &M.tri_v})
+                         &M.id, &M.counters, &M.comp_v, &M.parts, &M.pkey, &M.first, &M.tkey, &M.tidx, &M.tkey2,
+                         &M.tidx2, &M.tiles, &M.cub, &M.packed, &M.tri_a, &M.tri_v})
         n += b->cap;
     return n;
 }
@@ -377,26 +376,25 @@ int smb_engine_run_device(smb_engine* e, smb_batch_times* times, char* err, size
     if (ctl.cancelled()) return cancelled();
     ctl.report(SMB_STAGE_MESH, 0, surface);
     smb_batch_times t{};
-    rc = smb_run(e->res, 0, surface, e->batch, &t, err, errlen);
-    if (rc != SMB_OK) return rc;
-    if (ctl.cancelled()) return cancelled();
+    const bool fast = e->params.refine == SMB_REFINE_FAST;
+    // The warm start's candidates are the SES's features; a sphere field
+    // refines from the linear guess.
+    const smb_mlp* warm = e->warm && e->params.kind == SMB_SES ? e->warm : nullptr;
     e->rows_ready = false;
-    if (e->params.refine == SMB_REFINE_FAST) {
-        double ms = 0;
-        // The warm start's candidates are the SES's features; a sphere
-        // field refines from the linear guess.
-        rc = e->warm && e->params.kind == SMB_SES ? smb_refine_warm(e->res, e->batch, e->warm, &ms, err, errlen)
-                                                  : smb_refine(e->res, e->batch, &ms, err, errlen);
+    if (e->exact_device) {
+        rc = smb::run_vertices(e->res, 0, surface, e->batch, fast, warm, [&] { return ctl.cancelled(); }, &t, err,
+                               errlen);
         if (rc != SMB_OK) return rc;
-        t.total += ms;
-        if (e->exact_device) {
-            if ((rc = smb_place_fast(e->res, e->batch, &ms, err, errlen)) != SMB_OK) return rc;
+    } else {
+        if ((rc = smb_run(e->res, 0, surface, e->batch, &t, err, errlen)) != SMB_OK) return rc;
+        if (ctl.cancelled()) return cancelled();
+        if (fast) {
+            double ms = 0;
+            rc = warm ? smb_refine_warm(e->res, e->batch, warm, &ms, err, errlen)
+                      : smb_refine(e->res, e->batch, &ms, err, errlen);
+            if (rc != SMB_OK) return rc;
             t.total += ms;
         }
-    } else if (e->exact_device) {
-        double ms = 0;
-        if ((rc = smb_refine_exact(e->res, e->batch, &ms, err, errlen)) != SMB_OK) return rc;
-        t.total += ms;
     }
     e->times = t;
     if (times) *times = t;

@@ -597,6 +597,10 @@ void smb_resident_free(smb_resident* r) {
 
 size_t smb_resident_bytes(const smb_resident* r) { return r ? r->bytes : 0; }
 
+// Brick boxes up to this many bricks are classified in one go (16 bytes of
+// keys a brick, 1 MB at most).
+static constexpr uint32_t CLASSIFY_BLIND_MAX = 65536;
+
 int smb_classify(smb_resident* r, size_t* touched, size_t* surface, char* err, size_t errlen) {
     if (!r) return SMB_ERR_ARG;
     smb_device* d = r->dev;
@@ -652,32 +656,55 @@ int smb_classify(smb_resident* r, size_t* touched, size_t* surface, char* err, s
     launch_mark_touched(r->A, L, box, flags.as<uint32_t>(), errbuf.as<int>(), s);
     launch_scan(flags.as<uint32_t>(), nb, nullptr, list.as<uint32_t>(), tiles.as<unsigned long long>(),
                 tot.as<unsigned long long>(), s);
-    unsigned long long n_touched = 0;
+    unsigned long long n_touched = 0, n_surface = 0;
     int kerr = 0;
-    cudaMemcpyAsync(&n_touched, tot.p, 8, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(&kerr, errbuf.p, 4, cudaMemcpyDeviceToHost, s);
-    cudaError_t e = cudaStreamSynchronize(s);
+    cudaError_t e = cudaSuccess;
+    unsigned long long* d_tot = tot.as<unsigned long long>();
+    // A small box is classified without waiting for the counts: the kernels
+    // read them on the device and the keys have room for every brick.
+    const bool blind = nb <= CLASSIFY_BLIND_MAX;
+    auto read_touched = [&] {
+        cudaMemcpyAsync(&n_touched, d_tot, 8, cudaMemcpyDeviceToHost, s);
+        cudaMemcpyAsync(&kerr, errbuf.p, 4, cudaMemcpyDeviceToHost, s);
+    };
+    if (blind) {
+        e = mem_alloc(reinterpret_cast<void**>(&r->keys), size_t(nb) * sizeof(int4));
+    } else {
+        read_touched();
+        e = cudaStreamSynchronize(s);
+    }
+    if (e == cudaSuccess && !kerr) {
+        launch_classify_bricks(r->A, L, box, list.as<uint32_t>(), blind ? nb : uint32_t(n_touched),
+                               surf.as<uint32_t>(), s, nullptr, blind ? d_tot : nullptr);
+        launch_scan(surf.as<uint32_t>(), nb, nullptr, cells.as<uint32_t>(), tiles.as<unsigned long long>(), d_tot + 1, s);
+        if (blind) {
+            launch_cells_to_keys(box, cells.as<uint32_t>(), nb, r->keys, s, nullptr, d_tot + 1);
+            read_touched();
+            cudaEventRecord(e1, s);
+        }
+        cudaMemcpyAsync(&n_surface, d_tot + 1, 8, cudaMemcpyDeviceToHost, s);
+        e = cudaStreamSynchronize(s);
+        if (!blind) {
+            if (e == cudaSuccess && n_surface)
+                e = mem_alloc(reinterpret_cast<void**>(&r->keys), n_surface * sizeof(int4));
+            if (e == cudaSuccess)
+                launch_cells_to_keys(box, cells.as<uint32_t>(), uint32_t(n_surface), r->keys, s);
+            cudaEventRecord(e1, s);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        }
+    }
     if (e != cudaSuccess || kerr) {
         cleanup();
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
         if (e != cudaSuccess) return set_err(err, errlen, "classification failed: %s", cudaGetErrorString(e)), SMB_ERR_CUDA;
         return set_err(err, errlen, "coordinates too far from the origin for grid spacing %g", L.h), SMB_ERR_RANGE;
     }
-    launch_classify_bricks(r->A, L, box, list.as<uint32_t>(), uint32_t(n_touched), surf.as<uint32_t>(), s);
-    launch_scan(surf.as<uint32_t>(), nb, nullptr, cells.as<uint32_t>(), tiles.as<unsigned long long>(),
-                tot.as<unsigned long long>(), s);
-    unsigned long long n_surface = 0;
-    cudaMemcpyAsync(&n_surface, tot.p, 8, cudaMemcpyDeviceToHost, s);
-    e = cudaStreamSynchronize(s);
-    if (e == cudaSuccess && n_surface) e = mem_alloc(reinterpret_cast<void**>(&r->keys), n_surface * sizeof(int4));
-    if (e == cudaSuccess) launch_cells_to_keys(box, cells.as<uint32_t>(), uint32_t(n_surface), r->keys, s);
-    cudaEventRecord(e1, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     float ms = 0;
     cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     cleanup();
-    if (e != cudaSuccess) return set_err(err, errlen, "classification failed: %s", cudaGetErrorString(e)), SMB_ERR_CUDA;
     r->classify_ms = ms;
     r->n_touched = n_touched;
     r->n_bricks = uint32_t(n_surface);
@@ -697,6 +724,9 @@ int smb_resident_bricks(const smb_resident* r, int32_t* out, size_t cap) {
     return SMB_OK;
 }
 
+// A batch's page-locked words: counters, then totals and single words.
+static constexpr size_t BATCH_WORDS = 64, W_TOT = CNT_N, W_MISC = CNT_N + 8;
+
 int smb_batch_new(smb_resident* r, smb_batch** out, char* err, size_t errlen) {
     if (!r || !out) return set_err(err, errlen, "null argument"), SMB_ERR_ARG;
     CK(cudaSetDevice(r->dev->index));
@@ -704,6 +734,10 @@ int smb_batch_new(smb_resident* r, smb_batch** out, char* err, size_t errlen) {
     b->res = r;
     r->refs.fetch_add(1);
     for (auto& ev : b->ev) cudaEventCreate(&ev);
+    if (!(b->words = static_cast<unsigned long long*>(pinned_alloc(BATCH_WORDS * 8)))) {
+        smb_batch_free(b);
+        return set_err(err, errlen, "page-locked counter words"), SMB_ERR_MEMORY;
+    }
     {
         smb_device* d = r->dev;
         std::lock_guard<std::mutex> g(d->hint_mu);
@@ -720,6 +754,7 @@ void smb_batch_free(smb_batch* b) {
     cudaDeviceSynchronize();  // once for all buffers
     for (DBuf* p : b->bufs()) p->release_synced();
     for (auto& ev : b->ev) cudaEventDestroy(ev);
+    pinned_free(b->words);
     smb_resident* r = b->res;
     delete b;
     if (r->refs.fetch_sub(1) == 1 && r->freed.load()) destroy_resident(r);
@@ -729,9 +764,13 @@ void smb_batch_free(smb_batch* b) {
 // what they need.
 static constexpr size_t GATHER_SAMPLE_MIN = 8192;
 static constexpr uint32_t GATHER_SAMPLE_STRIDE = 64;
+// Up to this many sub-blocks (of the bricks, sampled or not) are gathered
+// without waiting for the number sampled.
+static constexpr size_t GATHER_BLIND_MAX = 12288;
 
-int smb_run(smb_resident* r, size_t first, size_t count, smb_batch* b, smb_batch_times* times, char* err,
-            size_t errlen) {
+// smb_run without the wait at its end (the marching cubes' fill is still
+// queued).
+static int run_queue(smb_resident* r, size_t first, size_t count, smb_batch* b, char* err, size_t errlen) {
     if (!r || !b || b->res != r) return set_err(err, errlen, "bad arguments"), SMB_ERR_ARG;
     if (!r->classified) return set_err(err, errlen, "smb_classify must run first"), SMB_ERR_STATE;
     if (first > r->n_bricks || count > r->n_bricks - first) return set_err(err, errlen, "brick range"), SMB_ERR_ARG;
@@ -746,10 +785,8 @@ int smb_run(smb_resident* r, size_t first, size_t count, smb_batch* b, smb_batch
     b->n_work = 0;
     b->n_edges = b->n_tris = 0;
     b->ids_words = 0;
-    if (count == 0) {
-        if (times) *times = smb_batch_times{};
-        return SMB_OK;
-    }
+    b->sum_ready = false;
+    if (count == 0) return SMB_OK;
     const int4* keys = r->keys + first;
     const size_t nsub = count * 8;
     b->window_ok = false;
@@ -770,16 +807,23 @@ int smb_run(smb_resident* r, size_t first, size_t count, smb_batch* b, smb_batch
     launch_scan(b->sampled.as<uint32_t>(), uint32_t(nsub), nullptr, b->work.as<uint32_t>(),
                 b->tiles.as<unsigned long long>(), b->totals.as<unsigned long long>(), s);
     cudaEventRecord(b->ev[1], s);
-    unsigned long long n_work = 0;
-    cudaMemcpyAsync(&n_work, b->totals.p, 8, cudaMemcpyDeviceToHost, s);
-    CK(cudaStreamSynchronize(s));
-    b->n_work = uint32_t(n_work);
+    // Few sub-blocks: gathered without waiting for their count, which the
+    // kernel reads on the device (pools and grid sized for all of them).
+    const bool blind = nsub <= GATHER_BLIND_MAX;
+    const unsigned long long* n_dev = blind ? b->totals.as<unsigned long long>() : nullptr;
+    unsigned long long n_work = nsub;
+    if (!blind) {
+        CK(cudaMemcpyAsync(b->words + W_TOT, b->totals.p, 8, cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        n_work = b->words[W_TOT];
+    }
 
     // (b) gather, with list memory grown and shared-memory caps raised as
     // needed (bit-identical results at any capacity).
     GatherCaps caps = b->caps;
     int warps = b->gather_warps;
-    unsigned long long cnt[CNT_N];
+    unsigned long long* cnt = b->words;
+    unsigned long long* tots = b->words + W_TOT;
     size_t want_ids = b->ids.cap / 4, want_pack = b->pack.cap / 16;
     double ids_per = 0, units_per = 0;
     {
@@ -787,8 +831,8 @@ int smb_run(smb_resident* r, size_t first, size_t count, smb_batch* b, smb_batch
         if (d->hint.b == L.b && d->hint.h == L.h && d->hint.probe == r->A.probe)
             ids_per = d->hint.ids_per, units_per = d->hint.units_per;
     }
-    if (n_work < GATHER_SAMPLE_MIN) {
-        // 48 KB a sub-block: at most 400 MB.
+    if (n_work < GATHER_SAMPLE_MIN || blind) {
+        // 48 KB a sub-block: at most 600 MB.
         want_ids = std::max<size_t>(want_ids, size_t(n_work) * 4096);
         want_pack = std::max<size_t>(want_pack, size_t(n_work) * 2048);
     } else if (!want_ids || !want_pack) {
@@ -834,10 +878,14 @@ int smb_run(smb_resident* r, size_t first, size_t count, smb_batch* b, smb_batch
         GatherOut O{b->rec.as<uint32_t>(), b->ids.as<uint32_t>(), b->pack.as<uint4>(), b->retry_a.as<uint32_t>(),
                     b->counters.as<unsigned long long>(), b->ids.cap / 4, b->pack.cap / 16, ~0ull, nullptr,
                     b->x_window.as<uint8_t>()};
-        cudaError_t e = launch_gather(r->A, L, keys, b->work.as<uint32_t>(), uint32_t(n_work), O, caps, warps, s);
+        cudaError_t e = launch_gather(r->A, L, keys, b->work.as<uint32_t>(), uint32_t(n_work), O, caps, warps, s,
+                                      nullptr, attempt ? nullptr : n_dev);
         if (e != cudaSuccess) return set_err(err, errlen, "gather launch: %s", cudaGetErrorString(e)), SMB_ERR_CUDA;
         CK(cudaMemcpyAsync(cnt, b->counters.p, CNT_N * 8, cudaMemcpyDeviceToHost, s));
+        if (!attempt) CK(cudaMemcpyAsync(tots, b->totals.p, 8, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
+        if (!attempt) n_work = tots[0];
+        b->n_work = uint32_t(n_work);
         if (cnt[CNT_NOMEM] && attempt < 4) {
             want_ids = size_t(cnt[CNT_IDS]) + size_t(cnt[CNT_IDS]) / 4 + 1024;
             want_pack = size_t(cnt[CNT_PACK]) + size_t(cnt[CNT_PACK]) / 4 + 1024;
@@ -924,13 +972,12 @@ int smb_run(smb_resident* r, size_t first, size_t count, smb_batch* b, smb_batch
                 b->tiles.as<unsigned long long>(), tot + 1, s, true);
     launch_scan(b->mc_counts.as<uint32_t>() + count, uint32_t(count), b->tri_off.as<uint32_t>(), nullptr,
                 b->tiles.as<unsigned long long>(), tot + 2, s, true);
-    unsigned long long t2[3];
-    CK(cudaMemcpyAsync(t2, tot, 24, cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(tots, tot, 24, cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(cnt, b->counters.p, CNT_N * 8, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     if (cnt[CNT_TIMEOUT]) return set_err(err, errlen, "a bounded wait for a bulk copy gave up"), SMB_ERR_TIMEOUT;
-    b->n_edges = size_t(t2[1]);
-    b->n_tris = size_t(t2[2]);
+    b->n_edges = size_t(tots[1]);
+    b->n_tris = size_t(tots[2]);
     if (b->n_edges >= (size_t(1) << 32) || b->n_tris >= (size_t(1) << 32))
         return set_err(err, errlen, "batch too large for 32-bit offsets"), SMB_ERR_MEMORY;
     if ((rc = b->edges.reserve(b->n_edges * 4, err, errlen)) || (rc = b->edge_vals.reserve(b->n_edges * 8, err, errlen)) ||
@@ -941,13 +988,34 @@ int smb_run(smb_resident* r, size_t first, size_t count, smb_batch* b, smb_batch
                   true, s);
     if (e != cudaSuccess) return set_err(err, errlen, "mc launch: %s", cudaGetErrorString(e)), SMB_ERR_CUDA;
     cudaEventRecord(b->ev[4], s);
-    CK(cudaStreamSynchronize(s));
-    if (times) {
-        float t[4];
-        for (int k = 0; k < 4; k++) cudaEventElapsedTime(&t[k], b->ev[k], b->ev[k + 1]);
-        times->substates = t[0], times->gather = t[1], times->sample = t[2], times->mc = t[3];
-        times->total = double(t[0]) + t[1] + t[2] + t[3];
-    }
+    return SMB_OK;
+}
+
+}  // extern "C"
+
+namespace smb {
+
+// Device times of the last run (waits for it).
+static void run_times(smb_batch* b, smb_batch_times* times) {
+    float t[4];
+    cudaEventSynchronize(b->ev[4]);
+    for (int k = 0; k < 4; k++) cudaEventElapsedTime(&t[k], b->ev[k], b->ev[k + 1]);
+    times->substates = t[0], times->gather = t[1], times->sample = t[2], times->mc = t[3];
+    times->total = double(t[0]) + t[1] + t[2] + t[3];
+}
+
+}  // namespace smb
+
+extern "C" {
+
+int smb_run(smb_resident* r, size_t first, size_t count, smb_batch* b, smb_batch_times* times, char* err,
+            size_t errlen) {
+    int rc = run_queue(r, first, count, b, err, errlen);
+    if (rc != SMB_OK) return rc;
+    if (times) *times = smb_batch_times{};
+    if (!count) return SMB_OK;
+    CK(cudaStreamSynchronize(r->dev->stream));
+    if (times) run_times(b, times);
     return SMB_OK;
 }
 
@@ -984,8 +1052,11 @@ static int exact_group(const smb_batch* b) {
 // refinement from them) or the feature pass alone (FEATURES: the rows'
 // features into e_x, evals = 1 marks the edges covered).
 enum { PASS_PLAIN = 0, PASS_WARM = 1, PASS_FEATURES = 2 };
-static int refine_pass(smb_resident* r, smb_batch* b, int pass, const smb_mlp* mlp, double* ms, char* err,
-                       size_t errlen, bool count = false) {
+// The pass queued (*queued; false when there is nothing to refine and it is
+// done); refine_done waits for it.
+static int refine_queue(smb_resident* r, smb_batch* b, int pass, const smb_mlp* mlp, bool* queued, char* err,
+                        size_t errlen, bool count = false) {
+    *queued = false;
     if (!r || !b || b->res != r) return set_err(err, errlen, "bad arguments"), SMB_ERR_ARG;
     if (!r->refine_ready) return set_err(err, errlen, "smb_resident_set_refinement must run first"), SMB_ERR_STATE;
     smb_device* d = r->dev;
@@ -1006,7 +1077,7 @@ static int refine_pass(smb_resident* r, smb_batch* b, int pass, const smb_mlp* m
         return rc;
     b->refined = false;
     b->refined_exact = false;
-    if (ms) *ms = 0;
+    b->sum_ready = false;
     if (ne == 0 || b->n_work == 0) {
         if (ne) CK(cudaMemsetAsync(b->e_evals.p, 0, ne * 4, s));
         CK(cudaStreamSynchronize(s));
@@ -1028,7 +1099,7 @@ static int refine_pass(smb_resident* r, smb_batch* b, int pass, const smb_mlp* m
         (rc = b->tiles.reserve(size_t(scan_tiles_needed(nw)) * 8, err, errlen)) ||
         (rc = b->x_ovf.reserve(size_t(nw) * 4 + 8, err, errlen)))
         return rc;
-    cudaEventRecord(b->ev[4], s);
+    cudaEventRecord(b->ev[5], s);
     CK(cudaMemsetAsync(b->e_evals.p, 0, ne * 4, s));
     unsigned long long* cnt = b->counters.as<unsigned long long>();
     CK(cudaMemsetAsync(cnt + CNT_TIMEOUT, 0, 8, s));
@@ -1062,16 +1133,37 @@ static int refine_pass(smb_resident* r, smb_batch* b, int pass, const smb_mlp* m
                                   d->smem_optin, s, nullptr, nullptr, b->x_ovf.as<uint32_t>(), b->r_region,
                                   refine_group(b), count);
     if (e != cudaSuccess) return set_err(err, errlen, "refine launch: %s", cudaGetErrorString(e)), SMB_ERR_CUDA;
-    cudaEventRecord(b->ev[5], s);
-    CK(cudaStreamSynchronize(s));
-    unsigned long long timeouts = 0;
-    CK(cudaMemcpy(&timeouts, cnt + CNT_TIMEOUT, 8, cudaMemcpyDeviceToHost));
-    if (timeouts) return set_err(err, errlen, "tensor-core wait timed out in %llu tiles", timeouts), SMB_ERR_CUDA;
-    float t = 0;
-    cudaEventElapsedTime(&t, b->ev[4], b->ev[5]);
-    if (ms) *ms = t;
+    cudaEventRecord(b->ev[6], s);
+    CK(cudaMemcpyAsync(b->words + W_MISC, cnt + CNT_TIMEOUT, 8, cudaMemcpyDeviceToHost, s));
+    *queued = true;
     b->refined = true;
     return SMB_OK;
+}
+
+// The end of a queued refinement, once the stream has been waited for.
+static int refine_done(smb_batch* b, double* ms, char* err, size_t errlen) {
+    if (b->words[W_MISC]) {
+        b->refined = false;
+        return set_err(err, errlen, "tensor-core wait timed out in %llu tiles", b->words[W_MISC]), SMB_ERR_CUDA;
+    }
+    float t = 0;
+    cudaEventElapsedTime(&t, b->ev[5], b->ev[6]);
+    if (ms) *ms = t;
+    return SMB_OK;
+}
+
+static int refine_pass(smb_resident* r, smb_batch* b, int pass, const smb_mlp* mlp, double* ms, char* err,
+                       size_t errlen, bool count = false) {
+    if (ms) *ms = 0;
+    bool queued = false;
+    int rc = refine_queue(r, b, pass, mlp, &queued, err, errlen, count);
+    if (rc != SMB_OK || !queued) return rc;
+    cudaError_t e = cudaStreamSynchronize(r->dev->stream);
+    if (e != cudaSuccess) {
+        b->refined = false;
+        return set_err(err, errlen, "refinement failed: %s", cudaGetErrorString(e)), SMB_ERR_CUDA;
+    }
+    return refine_done(b, ms, err, errlen);
 }
 
 int smb_refine(smb_resident* r, smb_batch* b, double* ms, char* err, size_t errlen) {
@@ -1238,6 +1330,7 @@ static int exact_pass(smb_resident* r, smb_batch* b, const uint8_t* mask, const 
         (rc = b->tiles.reserve(size_t(scan_tiles_needed(nw)) * 8, err, errlen)))
         return rc;
     b->x_block_items = 0;
+    b->sum_ready = false;
     if (!ne || !nw) return SMB_OK;
     unsigned long long* cnt = b->counters.as<unsigned long long>();
     ExactOut out{b->x_pos.as<float>(), b->x_nrm.as<float>(), b->x_atom.as<uint32_t>(), b->x_patch.as<uint8_t>(),
@@ -1252,12 +1345,24 @@ static int exact_pass(smb_resident* r, smb_batch* b, const uint8_t* mask, const 
                  cnt + CNT_QUEUE, b->rec.as<uint32_t>(), b->x_hint, gids, window};
     uint32_t over = 0, over_warp = 0;
     cudaError_t e;
-    // Waits for the passes so far; over: the entries the last one left.
-    auto wait = [&](const DBuf& list) {
-        if (cudaMemcpyAsync(&over_warp, b->x_ovf.p, 4, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
-            cudaMemcpyAsync(&over, list.p, 4, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
-            cudaStreamSynchronize(s) == cudaSuccess)
+    // Waits for the passes so far; over: the entries the last one left.  When
+    // it left none the vertices are done, and their summary (queued with the
+    // passes) is theirs.
+    auto wait = [&](const DBuf* list) {
+        unsigned long long* w = b->words + W_MISC;
+        w[2] = w[3] = 0;
+        cudaEventRecord(b->ev[8], s);
+        if ((count || launch_exact_summary(b->x_evals.as<uint32_t>(), ne, b->x_sum.as<unsigned long long>(), sms, s) ==
+                          cudaSuccess) &&
+            cudaMemcpyAsync(w, b->x_sum.p, 16, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
+            cudaMemcpyAsync(w + 2, b->x_ovf.p, 4, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
+            (!list || cudaMemcpyAsync(w + 3, list->p, 4, cudaMemcpyDeviceToHost, s) == cudaSuccess) &&
+            cudaStreamSynchronize(s) == cudaSuccess) {
+            over_warp = uint32_t(w[2]), over = uint32_t(w[3]);
+            b->sum[0] = w[0], b->sum[1] = w[1];
+            b->sum_ready = !count && !over;
             return int(SMB_OK);
+        }
         set_err(err, errlen, "exact refinement: %s", cudaGetErrorString(cudaGetLastError()));
         return int(SMB_ERR_CUDA);
     };
@@ -1265,7 +1370,7 @@ static int exact_pass(smb_resident* r, smb_batch* b, const uint8_t* mask, const 
         B.marked = true, B.list = marked, B.n_max = uint32_t(n_marked);
         e = launch_refine_exact_block(B, r->A, r->L, r->xa, out, sms, s);
         if (e != cudaSuccess) return set_err(err, errlen, "exact refine launch: %s", cudaGetErrorString(e)), SMB_ERR_CUDA;
-        if ((rc = wait(b->x_ovf2))) return rc;
+        if ((rc = wait(&b->x_ovf2))) return rc;
         if (!over) return SMB_OK;
         // Lists over a block's shared memory: every marked edge again, by
         // its sub-block's pass below (the results are the same).
@@ -1310,7 +1415,7 @@ static int exact_pass(smb_resident* r, smb_batch* b, const uint8_t* mask, const 
         if (e != cudaSuccess) return set_err(err, errlen, "exact refine launch: %s", cudaGetErrorString(e)), SMB_ERR_CUDA;
         I.ovf = b->x_ovf2.as<uint32_t>();
     }
-    if ((rc = wait(blocks ? b->x_ovf2 : b->x_ovf))) return rc;
+    if ((rc = wait(blocks ? &b->x_ovf2 : &b->x_ovf))) return rc;
     b->x_block_items = all_blocks ? nw : over_warp;
     if (!over) return SMB_OK;
     I.slab_bytes = exact_slab_bytes(sms);
@@ -1318,8 +1423,7 @@ static int exact_pass(smb_resident* r, smb_batch* b, const uint8_t* mask, const 
     I.slab = b->x_slab.as<unsigned char>();
     e = launch_refine_exact_slab(I, r->A, r->L, r->xa, out, sms, s);
     if (e != cudaSuccess) return set_err(err, errlen, "exact refine launch: %s", cudaGetErrorString(e)), SMB_ERR_CUDA;
-    CK(cudaStreamSynchronize(s));
-    return SMB_OK;
+    return wait(nullptr);
 }
 
 static int reserve_vertices(smb_batch* b, char* err, size_t errlen) {
@@ -1333,7 +1437,7 @@ static int reserve_vertices(smb_batch* b, char* err, size_t errlen) {
     return SMB_OK;
 }
 
-int smb_refine_exact(smb_resident* r, smb_batch* b, double* ms, char* err, size_t errlen) {
+static int exact_vertices(smb_resident* r, smb_batch* b, double* ms, char* err, size_t errlen) {
     if (!r || !b || b->res != r) return set_err(err, errlen, "bad arguments"), SMB_ERR_ARG;
     if (!r->exact_ready) return set_err(err, errlen, "smb_resident_set_exact must run first"), SMB_ERR_STATE;
     smb_device* d = r->dev;
@@ -1345,16 +1449,20 @@ int smb_refine_exact(smb_resident* r, smb_batch* b, double* ms, char* err, size_
     b->refined = false;
     b->x_exact_edges = b->n_edges;
     if (ms) *ms = 0;
-    cudaEventRecord(b->ev[4], s);
+    cudaEventRecord(b->ev[7], s);
+    cudaEventRecord(b->ev[8], s);
     if (b->n_edges) CK(cudaMemsetAsync(b->x_evals.p, 0, b->n_edges * 4, s));
     if ((rc = exact_pass(r, b, nullptr, nullptr, 0, err, errlen))) return rc;
-    cudaEventRecord(b->ev[5], s);
-    CK(cudaStreamSynchronize(s));
+    if (!b->sum_ready) CK(cudaStreamSynchronize(s));  // nothing was refined
     float t = 0;
-    cudaEventElapsedTime(&t, b->ev[4], b->ev[5]);
+    cudaEventElapsedTime(&t, b->ev[7], b->ev[8]);
     if (ms) *ms = t;
     b->refined_exact = true;
     return SMB_OK;
+}
+
+int smb_refine_exact(smb_resident* r, smb_batch* b, double* ms, char* err, size_t errlen) {
+    return exact_vertices(r, b, ms, err, errlen);
 }
 
 int smb_batch_count_exact_ops(smb_batch* b, unsigned long long* ops, char* err, size_t errlen) {
@@ -1369,7 +1477,10 @@ int smb_batch_count_exact_ops(smb_batch* b, unsigned long long* ops, char* err, 
     return SMB_OK;
 }
 
-int smb_place_fast(smb_resident* r, smb_batch* b, double* ms, char* err, size_t errlen) {
+// smb_place_fast; with refining, the f32 refinement before it may still be
+// queued (its end is checked here, with its time in *refine_ms).
+static int place_vertices(smb_resident* r, smb_batch* b, bool refining, double* refine_ms, double* ms, char* err,
+                          size_t errlen) {
     if (!r || !b || b->res != r) return set_err(err, errlen, "bad arguments"), SMB_ERR_ARG;
     if (!b->refined) return set_err(err, errlen, "smb_refine must run first"), SMB_ERR_STATE;
     if (!r->exact_ready) return set_err(err, errlen, "smb_resident_set_exact must run first"), SMB_ERR_STATE;
@@ -1382,8 +1493,9 @@ int smb_place_fast(smb_resident* r, smb_batch* b, double* ms, char* err, size_t 
         (rc = b->x_marked.reserve(ne * 4, err, errlen)))
         return rc;
     b->refined_exact = false;
+    b->sum_ready = false;
     if (ms) *ms = 0;
-    cudaEventRecord(b->ev[4], s);
+    cudaEventRecord(b->ev[7], s);
     ExactOut out{b->x_pos.as<float>(), b->x_nrm.as<float>(), b->x_atom.as<uint32_t>(), b->x_patch.as<uint8_t>(),
                  b->x_t.as<float>(), b->x_evals.as<uint32_t>()};
     unsigned long long* marked = b->x_sum.as<unsigned long long>();
@@ -1392,20 +1504,24 @@ int smb_place_fast(smb_resident* r, smb_batch* b, double* ms, char* err, size_t 
                                       b->e_feat.as<uint32_t>(), b->e_q.as<float>(), b->e_evals.as<uint32_t>(), out,
                                       b->x_mask.as<uint8_t>(), b->x_marked.as<uint32_t>(), marked, s);
     if (e != cudaSuccess) return set_err(err, errlen, "placement launch: %s", cudaGetErrorString(e)), SMB_ERR_CUDA;
-    unsigned long long n_marked = 0;
-    CK(cudaMemcpyAsync(&n_marked, marked, 8, cudaMemcpyDeviceToHost, s));
+    cudaEventRecord(b->ev[8], s);
+    CK(cudaMemcpyAsync(b->words + W_MISC + 1, marked, 8, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
+    if (refining && (rc = refine_done(b, refine_ms, err, errlen))) return rc;
+    const unsigned long long n_marked = b->words[W_MISC + 1];
     b->x_exact_edges = size_t(n_marked);
     if (n_marked && (rc = exact_pass(r, b, b->x_mask.as<uint8_t>(), b->x_marked.as<uint32_t>(), size_t(n_marked), err,
                                      errlen)))
         return rc;
-    cudaEventRecord(b->ev[5], s);
-    CK(cudaStreamSynchronize(s));
     float t = 0;
-    cudaEventElapsedTime(&t, b->ev[4], b->ev[5]);
+    cudaEventElapsedTime(&t, b->ev[7], b->ev[8]);
     if (ms) *ms = t;
     b->refined_exact = true;
     return SMB_OK;
+}
+
+int smb_place_fast(smb_resident* r, smb_batch* b, double* ms, char* err, size_t errlen) {
+    return place_vertices(r, b, false, nullptr, ms, err, errlen);
 }
 
 int smb_batch_vertices(const smb_batch* b, float* positions, float* normals, uint32_t* atoms, uint8_t* patches,
@@ -1431,8 +1547,9 @@ int smb_batch_exact_summary(const smb_batch* b, unsigned long long* evaluations,
     if (!b || !b->refined_exact) return SMB_ERR_STATE;
     smb_device* d = b->res->dev;
     if (cudaSetDevice(d->index) != cudaSuccess) return SMB_ERR_CUDA;
-    unsigned long long out[2] = {0, 0};
-    if (b->n_edges) {
+    unsigned long long out[2] = {b->sum[0], b->sum[1]};
+    if (!b->n_edges) out[0] = out[1] = 0;
+    if (b->n_edges && !b->sum_ready) {
         unsigned long long* sum = b->x_sum.as<unsigned long long>();
         if (!sum || launch_exact_summary(b->x_evals.as<uint32_t>(), b->n_edges, sum, d->info.multiprocessors,
                                          d->stream) != cudaSuccess ||
@@ -1588,3 +1705,33 @@ int smb_batch_mc(const smb_batch* b, uint32_t* edge_off, uint32_t* edges, float*
 }
 
 }  // extern "C"
+
+namespace smb {
+
+int run_vertices(smb_resident* r, size_t first, size_t count, smb_batch* b, bool fast, const smb_mlp* warm,
+                 const std::function<bool()>& stop, smb_batch_times* times, char* err, size_t errlen) {
+    *times = smb_batch_times{};
+    auto cancelled = [&] {
+        cudaStreamSynchronize(r->dev->stream);
+        return set_err(err, errlen, "cancelled"), SMB_ERR_CANCELLED;
+    };
+    int rc = run_queue(r, first, count, b, err, errlen);
+    if (rc != SMB_OK) return rc;
+    if (stop()) return cancelled();
+    double ms_refine = 0, ms = 0;
+    if (fast) {
+        bool queued = false;
+        if ((rc = refine_queue(r, b, warm ? PASS_WARM : PASS_PLAIN, warm, &queued, err, errlen)) != SMB_OK) return rc;
+        if (stop()) return cancelled();
+        rc = place_vertices(r, b, queued, &ms_refine, &ms, err, errlen);
+    } else {
+        rc = exact_vertices(r, b, &ms, err, errlen);
+    }
+    if (rc != SMB_OK) return rc;
+    if (count) run_times(b, times);
+    times->total += ms_refine + ms;
+    return SMB_OK;
+}
+
+}  // namespace smb
+

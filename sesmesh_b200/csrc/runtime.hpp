@@ -4,6 +4,7 @@
 #include <mutex>
 #include <cstddef>
 #include <cstdint>
+#include <functional>
 #include <vector>
 
 #include "../../include/sesmesh_b200.h"
@@ -45,6 +46,13 @@ void mem_device_close(int device);
 // frees them in (a garbage-collected host may finalize them in any order).
 void dev_retain(smb_device* d);
 void dev_release(smb_device* d);
+
+// The mesh stage of one batch run through its vertices (smb_run, then
+// smb_refine_exact, or smb_refine / smb_refine_warm and smb_place_fast)
+// without waiting for the device between them; stop() is asked between the
+// passes (SMB_ERR_CANCELLED).
+int run_vertices(smb_resident* r, size_t first, size_t count, smb_batch* b, bool fast, const smb_mlp* warm,
+                 const std::function<bool()>& stop, smb_batch_times* times, char* err, size_t errlen);
 
 // The warm-start MLP's device parameters and device (mlp.cu).
 struct MlpDev;
@@ -142,7 +150,12 @@ struct smb_batch {
     int gather_warps = 4;
     bool caps_seen = false;  // caps are those of an earlier run with these lattice and probe values
     bool use_tma = true;
-    cudaEvent_t ev[6] = {};
+    // Run 0..4 (sub-block states, gather, sampling, marching cubes), f32
+    // refinement 5..6, placement and exact refinement 7..8.
+    cudaEvent_t ev[9] = {};
+    unsigned long long* words = nullptr;  // page-locked: counters and totals read back
+    unsigned long long sum[2] = {0, 0};   // smb_batch_exact_summary's sums of the last vertices
+    bool sum_ready = false;               // sum is theirs
     std::vector<smb::DBuf*> bufs() {
         return {&rec, &sampled, &work, &retry_a, &retry_b, &values, &tiles, &totals, &counters,
                 &ids, &pack, &mc_counts, &edge_off, &tri_off, &edges, &edge_vals, &tris, &e_t, &e_feat, &e_q, &e_evals, &e_x, &w_feats, &w_start, &item_counts, &item_off, &item_edges,
