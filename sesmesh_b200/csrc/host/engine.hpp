@@ -61,7 +61,8 @@ struct smb_surface {
     Mesh mesh;
     std::vector<Component> comps;
     smb_surface_stats stats{};
-    smbh::ObjText obj;
+    smbh::ObjText obj;     // the OBJ text, once it had to be kept
+    smbh::ObjPlan obj_plan;  // its layout, once asked for
     // A mesh finished on the device stays in the page-locked block its
     // results came back in (view points into it); else view is of mesh.
     void* block = nullptr;

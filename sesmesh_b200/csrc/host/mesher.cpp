@@ -800,15 +800,11 @@ static inline size_t u64_len(uint64_t v) {
 // of each chunk, then each chunk formatted straight into its place, so the
 // text is written once into one buffer (no intermediate copies).
 static const char OBJ_HEAD[] = "# sesmesh 1.3.2\no ses\n";
-constexpr size_t OBJ_CH = 1 << 15;
+// Lines of a chunk: small enough that 16 threads share a mesh of 100,000
+// vertices evenly.
+constexpr size_t OBJ_CH = 1 << 12;
 
-struct ObjPlan {
-    std::vector<size_t> at;  // chunk start offsets: v chunks, vn chunks, f chunks, then the end
-    size_t nvc = 0, nfc = 0;
-    bool normals = false;
-};
-
-static ObjPlan obj_plan(const MeshRef& m, int precision, bool normals) {
+ObjPlan obj_plan(const MeshRef& m, int precision, bool normals) {
     ObjPlan P;
     P.normals = normals && m.nrm;
     const size_t nv = m.nv, nt = m.nt;
@@ -843,7 +839,7 @@ static ObjPlan obj_plan(const MeshRef& m, int precision, bool normals) {
     return P;
 }
 
-static void obj_fill(const MeshRef& m, int precision, const ObjPlan& P, char* out) {
+void obj_fill(const MeshRef& m, int precision, const ObjPlan& P, char* out) {
     std::memcpy(out, OBJ_HEAD, sizeof OBJ_HEAD - 1);
     const size_t nv = m.nv, nt = m.nt;
     const size_t nvec = P.normals ? 2 : 1, nch = nvec * P.nvc + P.nfc;

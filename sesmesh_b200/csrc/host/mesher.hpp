@@ -141,6 +141,16 @@ struct MeshRef {
 
 std::string obj_text(const MeshRef& m, int precision = 4, bool normals = true);
 // The same text in a buffer that is written once (not zero-filled first).
+// The places of an OBJ text's chunks of lines (offsets of the v, vn and f
+// chunks, then the text's size), and the text written at them.
+struct ObjPlan {
+    std::vector<size_t> at;
+    size_t nvc = 0, nfc = 0;
+    bool normals = false;
+    size_t size() const { return at.empty() ? 0 : at.back(); }
+};
+ObjPlan obj_plan(const MeshRef& m, int precision = 4, bool normals = true);
+void obj_fill(const MeshRef& m, int precision, const ObjPlan& P, char* out);
 struct ObjText {
     std::unique_ptr<char[]> data;
     size_t size = 0;

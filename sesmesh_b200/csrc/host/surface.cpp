@@ -36,6 +36,22 @@ void set_err(char* err, size_t len, const char* fmt, ...) {
     va_end(ap);
 }
 
+// memcpy on the host threads where it is worth their start: a fresh
+// destination's page faults, which the copy mostly waits for, are then taken
+// by all of them.
+void copy_parallel(void* dst, const void* src, size_t bytes) {
+    constexpr size_t PIECE = size_t(1) << 20;
+    if (bytes < 8 * PIECE) {
+        std::memcpy(dst, src, bytes);
+        return;
+    }
+    const size_t n = (bytes + PIECE - 1) / PIECE;
+    parallel_for(n, [&](size_t k, int) {
+        std::memcpy(static_cast<char*>(dst) + k * PIECE, static_cast<const char*>(src) + k * PIECE,
+                    std::min(PIECE, bytes - k * PIECE));
+    });
+}
+
 }  // namespace
 
 // Host stages of one structure after its device run: placement of the
@@ -700,7 +716,7 @@ int smb_surface_mesh(const smb_surface* s, float* pos, float* nrm, uint32_t* tri
     if (!s) return SMB_ERR_ARG;
     const smbh::MeshRef m = s->ref();
     auto copy = [](void* dst, const void* src, size_t bytes) {
-        if (dst && src && bytes) std::memcpy(dst, src, bytes);
+        if (dst && src && bytes) copy_parallel(dst, src, bytes);
     };
     copy(pos, m.pos, m.nv * 12);
     copy(nrm, m.nrm, m.nv * 12);
@@ -726,9 +742,16 @@ int smb_surface_arrays(const smb_surface* s, const float** pos, const float** nr
 
 size_t smb_surface_obj(smb_surface* s, char* out, size_t cap) {
     if (!s) return 0;
+    if (s->obj_plan.at.empty()) s->obj_plan = obj_plan(s->ref());
+    const size_t n = s->obj_plan.size();
+    if (!out) return n;
+    if (s->obj.empty() && cap >= n) {  // straight into the caller's buffer
+        obj_fill(s->ref(), 4, s->obj_plan, out);
+        return n;
+    }
     if (s->obj.empty()) s->obj = obj_text_buffer(s->ref());
-    if (out) std::memcpy(out, s->obj.data.get(), s->obj.size < cap ? s->obj.size : cap);
-    return s->obj.size;
+    copy_parallel(out, s->obj.data.get(), std::min(n, cap));
+    return n;
 }
 
 int smb_surface_write_obj(smb_surface* s, const char* path, char* err, size_t errlen) {

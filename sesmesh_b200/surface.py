@@ -73,6 +73,10 @@ class SurfaceParams:
         return p
 
 
+_new_bytes = C.pythonapi.PyBytes_FromStringAndSize
+_new_bytes.restype, _new_bytes.argtypes = C.py_object, [C.c_char_p, C.c_ssize_t]
+
+
 class _SurfaceHandle:
     """Owns one smb_surface; freed when the output and every array view of
     it are gone."""
@@ -105,7 +109,7 @@ class SurfaceOutput:
         self.stats = {name: getattr(st, name) for name, _ in st._fields_}
         self._arrays = None
         if not owned:
-            self._arrays = {k: v.copy() for k, v in self._views().items()}
+            self._arrays = self._copies()
 
     def _views(self):
         nv, nt = self.stats["vertices"], self.stats["triangles"]
@@ -126,6 +130,18 @@ class SurfaceOutput:
             out[name] = a
         return out
 
+    def _copies(self):
+        """The mesh in arrays of its own (copied by the library's threads)."""
+        nv, nt = self.stats["vertices"], self.stats["triangles"]
+        out = {}
+        for name, ct, dt, width in self._ARRAYS:
+            rows = nt if name == "triangles" else nv
+            out[name] = np.empty((rows, width) if width else (rows,), dt)
+        lib().smb_surface_mesh(self._h, *[_p(out[name], ct) for name, ct, _, _ in self._ARRAYS[:2]],
+                               *[_p(out[k], C.c_uint32) for k in ("triangles", "vertex_atom")],
+                               _p(out["vertex_patch"], C.c_uint8), _p(out["vertex_component"], C.c_uint32))
+        return out
+
     def _array(self, name):
         if self._arrays is None:
             if self._h is None:
@@ -143,9 +159,14 @@ class SurfaceOutput:
     def obj(self):
         """OBJ bytes with the default options (export/obj.rs:37-73)."""
         n = lib().smb_surface_obj(self._h, None, 0)
-        buf = C.create_string_buffer(n)
-        lib().smb_surface_obj(self._h, buf, n)
-        return buf.raw[:n]
+        if n < 2:  # bytes objects of 0 and 1 bytes are shared
+            buf = C.create_string_buffer(n)
+            lib().smb_surface_obj(self._h, buf, n)
+            return buf.raw[:n]
+        # Formatted into the bytes object itself, which nothing else holds yet.
+        text = _new_bytes(None, n)
+        lib().smb_surface_obj(self._h, text, n)
+        return text
 
     def write_obj(self, path):
         err = C.create_string_buffer(512)
