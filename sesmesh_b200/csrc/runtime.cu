@@ -872,8 +872,20 @@ static int run_queue(smb_resident* r, size_t first, size_t count, smb_batch* b, 
         want_pack = std::max<size_t>(size_t(units_per * 1.25 * double(n_work)), size_t(n_work) * 128);
     }
     for (int attempt = 0;; attempt++) {
-        if ((rc = b->ids.reserve(want_ids * 4, err, errlen)) || (rc = b->pack.reserve(want_pack * 16, err, errlen)))
-            return rc;
+        auto pools = [&] {
+            const int r1 = b->ids.reserve(want_ids * 4, err, errlen);
+            return r1 ? r1 : b->pack.reserve(want_pack * 16, err, errlen);
+        };
+        rc = pools();
+        if (rc == SMB_ERR_MEMORY && !attempt) {
+            // No room for a generous first guess: a small one, whose pass
+            // counts what the lists need.
+            cudaGetLastError();
+            b->ids.release(), b->pack.release();
+            want_ids = size_t(n_work) * 256, want_pack = size_t(n_work) * 128;
+            rc = pools();
+        }
+        if (rc) return rc;
         CK(cudaMemsetAsync(b->counters.p, 0, CNT_N * 8, s));
         GatherOut O{b->rec.as<uint32_t>(), b->ids.as<uint32_t>(), b->pack.as<uint4>(), b->retry_a.as<uint32_t>(),
                     b->counters.as<unsigned long long>(), b->ids.cap / 4, b->pack.cap / 16, ~0ull, nullptr,
