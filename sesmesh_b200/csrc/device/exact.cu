@@ -553,16 +553,48 @@ struct XEval {
     uint32_t kind, id;
 };
 
+// How far around an evaluated point its nearest candidate is certain to stay
+// the nearest one, if it stays unblocked: within r of it (r <= 0: unknown).
+// Each candidate's value is 1-Lipschitz, so one whose value lies m above the
+// winner's cannot pass it within m / 2; a blocked candidate stays blocked
+// while its projection, which moves R / (len - move) times as far as the
+// point, cannot leave the blocker it lies `depth` inside of.  pos: the
+// winner's place in its list; in_k: the sphere that contains the point.
+// Kept in f32, rounded towards smaller r.
+struct XSafe {
+    float r;
+    uint32_t kind, pos, in_k;
+};
+
+__device__ __forceinline__ float x_sqrt_below(double d2) {
+    float r;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(__double2float_rd(d2)));
+    return r * 0.999999f;
+}
+
+// The move below which a projection from distance len onto radius R stays
+// inside a blocker of radius T, d2 the squared distance from its centre.
+__device__ __forceinline__ float x_blocked_within(double d2, double T, double len, double R) {
+    if (!(T > 0.0)) return 0.0f;
+    const float depth = __fdividef(__double2float_rd(T * T - d2), 2.00001f * float(T));  // of T - d >= (T^2 - d2) / 2T
+    return depth * __fdividef(float(len), float(R) + depth);
+}
+
+__device__ __forceinline__ float x_safe_radius(float blocked, float m, double best) {
+    return fminf(blocked * 0.999f, 0.5f * (m - __double2float_ru(best))) - 1e-6f;
+}
+
 // eval_local (point.rs:686-738) against the ball's lists: value, feature and
 // closest point.  COUNT: adds the f64 arithmetic operations executed to ops
 // (sqrt and division one each; compares, selects, fabs not counted): 9 per
 // inside sphere tested; if inside, 1, then 10 per S candidate visited (+7
 // for the projection, +10 per blocker tested), 26 per C candidate (+9 or +6,
 // +10 per blocker), 9 per SAS vertex, 1 final.
-template <bool COUNT = false>
+template <bool COUNT, bool SAFE>
 __device__ __forceinline__ XEval x_eval(const XView& v, const double* circ, double probe, double band, double x,
-                                        double y, double z, unsigned long long* ops = nullptr) {
+                                        double y, double z, XSafe& safe, unsigned long long* ops = nullptr) {
     XEval e;
+    safe.r = 0.0f;
     e.qx = x, e.qy = y, e.qz = z, e.id = 0;
     bool inside = false;
     unsigned long long n_ops = 0;
@@ -571,6 +603,7 @@ __device__ __forceinline__ XEval x_eval(const XView& v, const double* circ, doub
         if (COUNT) n_ops += 9;
         if (sqrt_lt(sq3(x, y, z, c.x, c.y, c.z), c.w)) {
             inside = true;
+            safe.in_k = k;
             break;
         }
     }
@@ -582,6 +615,7 @@ __device__ __forceinline__ XEval x_eval(const XView& v, const double* circ, doub
     double best = probe + band;
     if (COUNT) n_ops += 1;
     e.kind = XF_BEYOND;
+    float m = __double2float_rd(best), blocked = 1e30f;  // the other values, the blocked projections
     // Pruning at this point: a candidate's value here is at least its value
     // at the ball's centre minus |x - centre| (each is 1-Lipschitz), so with
     // slack = rho - |x - centre| (less a 1e-12 rounding margin, at least 0)
@@ -590,13 +624,21 @@ __device__ __forceinline__ XEval x_eval(const XView& v, const double* circ, doub
     // below best, so the result is the unpruned one.
     const double ddx = x - v.cx, ddy = y - v.cy, ddz = z - v.cz;
     const double slack = fmax(v.rho - sqrt(ddx * ddx + ddy * ddy + ddz * ddz) - 1e-12, 0.0);
-    for (uint32_t i = 0; i < v.ns && v.s_key[i] < best - slack; i++) {
+    for (uint32_t i = 0; i < v.ns; i++) {
+        const double key = v.s_key[i];
+        if (!(key < best - slack)) {
+            if (SAFE) m = fminf(m, __double2float_rd(key + slack));
+            break;
+        }
         const double4 c = v.s_c[i];
         const double vx = x - c.x, vy = y - c.y, vz = z - c.z;
         const double len = sqrt(vx * vx + vy * vy + vz * vz);
         const double lb = fabs(len - c.w);
         if (COUNT) n_ops += 10;
-        if (lb >= best || len < 1e-12) continue;
+        if (lb >= best || len < 1e-12) {
+            if (SAFE) m = fminf(m, __double2float_rd(lb));
+            continue;
+        }
         const double s = c.w / len;
         const double qx = c.x + vx * s, qy = c.y + vy * s, qz = c.z + vz * s;
         if (COUNT) n_ops += 7;
@@ -604,22 +646,35 @@ __device__ __forceinline__ XEval x_eval(const XView& v, const double* circ, doub
         for (uint32_t p = v.s_off[i], pe = v.s_off[i + 1]; p < pe; p++) {
             const double4 k = v.near_c[v.s_blk[p]];
             if (COUNT) n_ops += 10;
-            if (!sqrt_ge(sq3(qx, qy, qz, k.x, k.y, k.z), k.w - X_EPS)) {
+            const double d2 = sq3(qx, qy, qz, k.x, k.y, k.z);
+            if (!sqrt_ge(d2, k.w - X_EPS)) {
                 free = false;
+                if (SAFE) blocked = fminf(blocked, x_blocked_within(d2, k.w - X_EPS, len, c.w));
                 break;
             }
         }
-        if (free) best = lb, e.kind = XF_SPHERE, e.id = v.s_id[i], e.qx = qx, e.qy = qy, e.qz = qz;
+        if (free) {
+            if (SAFE) m = fminf(m, __double2float_rd(best));
+            best = lb, e.kind = XF_SPHERE, e.id = v.s_id[i], e.qx = qx, e.qy = qy, e.qz = qz, safe.pos = i;
+        }
     }
-    for (uint32_t i = 0; i < v.nc && v.c_key[i] < best - slack; i++) {
-        const double4 m = v.c_m[i], u = v.c_u[i];
-        const double yx = x - m.x, yy = y - m.y, yz = z - m.z;
+    for (uint32_t i = 0; i < v.nc; i++) {
+        const double key = v.c_key[i];
+        if (!(key < best - slack)) {
+            if (SAFE) m = fminf(m, __double2float_rd(key + slack));
+            break;
+        }
+        const double4 o = v.c_m[i], u = v.c_u[i];
+        const double yx = x - o.x, yy = y - o.y, yz = z - o.z;
         const double along = yx * u.x + yy * u.y + yz * u.z;
         const double wx = yx - u.x * along, wy = yy - u.y * along, wz = yz - u.z * along;
         const double wl = sqrt(wx * wx + wy * wy + wz * wz);
-        const double dist2 = along * along + (wl - m.w) * (wl - m.w);
+        const double dist2 = along * along + (wl - o.w) * (wl - o.w);
         if (COUNT) n_ops += 26;
-        if (sqrt_ge(dist2, best)) continue;
+        if (sqrt_ge(dist2, best)) {
+            if (SAFE) m = fminf(m, x_sqrt_below(dist2));
+            continue;
+        }
         const double dist = sqrt(dist2);
         double dx, dy, dz;
         if (wl > 1e-12) {
@@ -629,29 +684,97 @@ __device__ __forceinline__ XEval x_eval(const XView& v, const double* circ, doub
             const double* C = circ + 12 * size_t(v.c_id[i]);
             dx = u.w, dy = C[7], dz = C[8];
         }
-        const double qx = m.x + dx * m.w, qy = m.y + dy * m.w, qz = m.z + dz * m.w;
+        const double qx = o.x + dx * o.w, qy = o.y + dy * o.w, qz = o.z + dz * o.w;
         if (COUNT) n_ops += 6;
         bool free = true;
         for (uint32_t p = v.c_off[i], pe = v.c_off[i + 1]; p < pe; p++) {
             const double4 k = v.near_c[v.c_blk[p]];
             if (COUNT) n_ops += 10;
-            if (!sqrt_ge(sq3(qx, qy, qz, k.x, k.y, k.z), k.w - X_EPS)) {
+            const double d2 = sq3(qx, qy, qz, k.x, k.y, k.z);
+            if (!sqrt_ge(d2, k.w - X_EPS)) {
                 free = false;
+                if (SAFE) blocked = fminf(blocked, x_blocked_within(d2, k.w - X_EPS, wl, o.w));
                 break;
             }
         }
-        if (free) best = dist, e.kind = XF_CIRCLE, e.id = v.c_id[i], e.qx = qx, e.qy = qy, e.qz = qz;
+        if (free) {
+            if (SAFE) m = fminf(m, __double2float_rd(best));
+            best = dist, e.kind = XF_CIRCLE, e.id = v.c_id[i], e.qx = qx, e.qy = qy, e.qz = qz, safe.pos = i;
+        }
     }
-    for (uint32_t i = 0; i < v.nv && v.v_key[i] < best - slack; i++) {
+    for (uint32_t i = 0; i < v.nv; i++) {
+        const double key = v.v_key[i];
+        if (!(key < best - slack)) {
+            if (SAFE) m = fminf(m, __double2float_rd(key + slack));
+            break;
+        }
         const double4 p = v.v_p[i];
         const double d2 = sq3(x, y, z, p.x, p.y, p.z);
         if (COUNT) n_ops += 9;
-        if (!sqrt_lt(d2, best)) continue;
-        best = sqrt(d2), e.kind = XF_VERTEX, e.id = v.v_id[i], e.qx = p.x, e.qy = p.y, e.qz = p.z;
+        if (!sqrt_lt(d2, best)) {
+            if (SAFE) m = fminf(m, x_sqrt_below(d2));
+            continue;
+        }
+        if (SAFE) m = fminf(m, __double2float_rd(best));
+        best = sqrt(d2), e.kind = XF_VERTEX, e.id = v.v_id[i], e.qx = p.x, e.qy = p.y, e.qz = p.z, safe.pos = i;
     }
     if (COUNT) *ops += n_ops + 1;
     e.value = probe - best;
+    safe.kind = e.kind;
+    if (SAFE && e.kind != XF_BEYOND) safe.r = x_safe_radius(blocked, m, best);
     return e;
+}
+
+// x_eval at a point within safe.r of the point safe was taken at, from its
+// winner alone: false where the winner does not hold (the walk then
+// decides).  By a group of RG lanes (RG = 1: a lane), which share its
+// blockers.
+template <int RG>
+__device__ __forceinline__ bool x_eval_again(const XView& v, const double* circ, double probe, double band, double x,
+                                             double y, double z, const XSafe& safe, XEval& e, int gl, uint32_t gm) {
+    const double4 in = v.in_c[safe.in_k];
+    if (!sqrt_lt(sq3(x, y, z, in.x, in.y, in.z), in.w)) return false;
+    const double best = probe + band;
+    const uint32_t i = safe.pos;
+    e.kind = safe.kind;
+    if (safe.kind == XF_VERTEX) {
+        const double4 p = v.v_p[i];
+        const double d2 = sq3(x, y, z, p.x, p.y, p.z);
+        if (!sqrt_lt(d2, best)) return false;
+        e.value = probe - sqrt(d2), e.id = v.v_id[i], e.qx = p.x, e.qy = p.y, e.qz = p.z;
+        return true;
+    }
+    const uint32_t *off, *blk;
+    if (safe.kind == XF_SPHERE) {
+        const double4 c = v.s_c[i];
+        const double vx = x - c.x, vy = y - c.y, vz = z - c.z;
+        const double len = sqrt(vx * vx + vy * vy + vz * vz);
+        const double lb = fabs(len - c.w);
+        if (lb >= best || len < 1e-12) return false;
+        const double s = c.w / len;
+        e.value = probe - lb, e.id = v.s_id[i];
+        e.qx = c.x + vx * s, e.qy = c.y + vy * s, e.qz = c.z + vz * s;
+        off = v.s_off, blk = v.s_blk;
+    } else {
+        const double4 o = v.c_m[i], u = v.c_u[i];
+        const double yx = x - o.x, yy = y - o.y, yz = z - o.z;
+        const double along = yx * u.x + yy * u.y + yz * u.z;
+        const double wx = yx - u.x * along, wy = yy - u.y * along, wz = yz - u.z * along;
+        const double wl = sqrt(wx * wx + wy * wy + wz * wz);
+        const double dist2 = along * along + (wl - o.w) * (wl - o.w);
+        // On the axis (where the walk takes e1 for the direction): left to it.
+        if (sqrt_ge(dist2, best) || !(wl > 1e-12)) return false;
+        e.value = probe - sqrt(dist2), e.id = v.c_id[i];
+        const double dx = wx / wl, dy = wy / wl, dz = wz / wl;
+        e.qx = o.x + dx * o.w, e.qy = o.y + dy * o.w, e.qz = o.z + dz * o.w;
+        off = v.c_off, blk = v.c_blk;
+    }
+    bool hit = false;
+    for (uint32_t p = off[i] + uint32_t(gl), pe = off[i + 1]; p < pe && !hit; p += RG) {
+        const double4 k = v.near_c[blk[p]];
+        hit = !sqrt_ge(sq3(e.qx, e.qy, e.qz, k.x, k.y, k.z), k.w - X_EPS);
+    }
+    return !(RG == 1 ? hit : __any_sync(gm, hit));
 }
 
 // x_eval by a group of RG lanes that all hold the same point: the lanes
@@ -670,12 +793,14 @@ __device__ __forceinline__ void x_argmin(uint32_t gm, double& v, int& i) {
     }
 }
 
-template <int RG>
+template <int RG, bool SAFE>
 __device__ __forceinline__ XEval x_eval_group(const XView& v, const double* circ, double probe, double band, double x,
-                                              double y, double z, int gl, uint32_t gm) {
+                                              double y, double z, XSafe& safe, int gl, uint32_t gm) {
     const double inf = __longlong_as_double(0x7ff0000000000000LL);
     XEval e;
     e.qx = x, e.qy = y, e.qz = z, e.id = 0;
+    safe.r = 0.0f;
+    const int g0 = int(threadIdx.x & 31) & ~(RG - 1);
     bool inside = false;
     for (uint32_t k0 = 0; k0 < v.ni; k0 += RG) {
         const uint32_t k = k0 + gl;
@@ -684,8 +809,10 @@ __device__ __forceinline__ XEval x_eval_group(const XView& v, const double* circ
             const double4 c = v.in_c[k];
             in = sqrt_lt(sq3(x, y, z, c.x, c.y, c.z), c.w);
         }
-        if (__any_sync(gm, in)) {
+        const uint32_t at = __ballot_sync(gm, in);
+        if (at) {
             inside = true;
+            safe.in_k = k0 + uint32_t(__ffs(int(at)) - 1 - g0);
             break;
         }
     }
@@ -695,13 +822,20 @@ __device__ __forceinline__ XEval x_eval_group(const XView& v, const double* circ
     }
     double best = probe + band;
     e.kind = XF_BEYOND;
+    // As in x_eval, over the lane's own candidates.
+    float m = __double2float_rd(best), blocked = 1e30f;
     const double ddx = x - v.cx, ddy = y - v.cy, ddz = z - v.cz;
     const double slack = fmax(v.rho - sqrt(ddx * ddx + ddy * ddy + ddz * ddz) - 1e-12, 0.0);
-    const int g0 = int(threadIdx.x & 31) & ~(RG - 1);
-    for (uint32_t i0 = 0; i0 < v.ns && v.s_key[i0] < best - slack; i0 += RG) {
+    for (uint32_t i0 = 0; i0 < v.ns; i0 += RG) {
+        if (!(v.s_key[i0] < best - slack)) {
+            if (SAFE) m = fminf(m, __double2float_rd(v.s_key[i0] + slack));
+            break;
+        }
         const uint32_t i = i0 + gl;
         double val = inf, qx = 0.0, qy = 0.0, qz = 0.0;
-        if (i < v.ns && v.s_key[i] < best - slack) {
+        if (i < v.ns && !(v.s_key[i] < best - slack)) {
+            if (SAFE) m = fminf(m, __double2float_rd(v.s_key[i] + slack));
+        } else if (i < v.ns) {
             const double4 c = v.s_c[i];
             const double vx = x - c.x, vy = y - c.y, vz = z - c.z;
             const double len = sqrt(vx * vx + vy * vy + vz * vz);
@@ -712,32 +846,46 @@ __device__ __forceinline__ XEval x_eval_group(const XView& v, const double* circ
                 bool free = true;
                 for (uint32_t p = v.s_off[i], pe = v.s_off[i + 1]; p < pe; p++) {
                     const double4 k = v.near_c[v.s_blk[p]];
-                    if (!sqrt_ge(sq3(qx, qy, qz, k.x, k.y, k.z), k.w - X_EPS)) {
+                    const double d2 = sq3(qx, qy, qz, k.x, k.y, k.z);
+                    if (!sqrt_ge(d2, k.w - X_EPS)) {
                         free = false;
+                        if (SAFE) blocked = fminf(blocked, x_blocked_within(d2, k.w - X_EPS, len, c.w));
                         break;
                     }
                 }
                 if (free) val = lb;
+            } else {
+                if (SAFE) m = fminf(m, __double2float_rd(lb));
             }
         }
+        const float own = __double2float_rd(val);
         int w = int(i);
         x_argmin<RG>(gm, val, w);
+        if (SAFE && (!(val < best) || w != int(i))) m = fminf(m, own);
         if (val < best) {
+            if (SAFE) m = fminf(m, __double2float_rd(best));
+            safe.pos = uint32_t(w);
             const int src = g0 + (w - int(i0));
             best = val, e.kind = XF_SPHERE, e.id = v.s_id[w];
             e.qx = __shfl_sync(gm, qx, src), e.qy = __shfl_sync(gm, qy, src), e.qz = __shfl_sync(gm, qz, src);
         }
     }
-    for (uint32_t i0 = 0; i0 < v.nc && v.c_key[i0] < best - slack; i0 += RG) {
+    for (uint32_t i0 = 0; i0 < v.nc; i0 += RG) {
+        if (!(v.c_key[i0] < best - slack)) {
+            if (SAFE) m = fminf(m, __double2float_rd(v.c_key[i0] + slack));
+            break;
+        }
         const uint32_t i = i0 + gl;
         double val = inf, qx = 0.0, qy = 0.0, qz = 0.0;
-        if (i < v.nc && v.c_key[i] < best - slack) {
-            const double4 m = v.c_m[i], u = v.c_u[i];
-            const double yx = x - m.x, yy = y - m.y, yz = z - m.z;
+        if (i < v.nc && !(v.c_key[i] < best - slack)) {
+            if (SAFE) m = fminf(m, __double2float_rd(v.c_key[i] + slack));
+        } else if (i < v.nc) {
+            const double4 o = v.c_m[i], u = v.c_u[i];
+            const double yx = x - o.x, yy = y - o.y, yz = z - o.z;
             const double along = yx * u.x + yy * u.y + yz * u.z;
             const double wx = yx - u.x * along, wy = yy - u.y * along, wz = yz - u.z * along;
             const double wl = sqrt(wx * wx + wy * wy + wz * wz);
-            const double dist2 = along * along + (wl - m.w) * (wl - m.w);
+            const double dist2 = along * along + (wl - o.w) * (wl - o.w);
             if (!sqrt_ge(dist2, best)) {
                 const double dist = sqrt(dist2);
                 double dx, dy, dz;
@@ -747,42 +895,67 @@ __device__ __forceinline__ XEval x_eval_group(const XView& v, const double* circ
                     const double* C = circ + 12 * size_t(v.c_id[i]);
                     dx = u.w, dy = C[7], dz = C[8];
                 }
-                qx = m.x + dx * m.w, qy = m.y + dy * m.w, qz = m.z + dz * m.w;
+                qx = o.x + dx * o.w, qy = o.y + dy * o.w, qz = o.z + dz * o.w;
                 bool free = true;
                 for (uint32_t p = v.c_off[i], pe = v.c_off[i + 1]; p < pe; p++) {
                     const double4 k = v.near_c[v.c_blk[p]];
-                    if (!sqrt_ge(sq3(qx, qy, qz, k.x, k.y, k.z), k.w - X_EPS)) {
+                    const double d2 = sq3(qx, qy, qz, k.x, k.y, k.z);
+                    if (!sqrt_ge(d2, k.w - X_EPS)) {
                         free = false;
+                        if (SAFE) blocked = fminf(blocked, x_blocked_within(d2, k.w - X_EPS, wl, o.w));
                         break;
                     }
                 }
                 if (free) val = dist;
+            } else {
+                if (SAFE) m = fminf(m, x_sqrt_below(dist2));
             }
         }
+        const float own = __double2float_rd(val);
         int w = int(i);
         x_argmin<RG>(gm, val, w);
+        if (SAFE && (!(val < best) || w != int(i))) m = fminf(m, own);
         if (val < best) {
+            if (SAFE) m = fminf(m, __double2float_rd(best));
+            safe.pos = uint32_t(w);
             const int src = g0 + (w - int(i0));
             best = val, e.kind = XF_CIRCLE, e.id = v.c_id[w];
             e.qx = __shfl_sync(gm, qx, src), e.qy = __shfl_sync(gm, qy, src), e.qz = __shfl_sync(gm, qz, src);
         }
     }
-    for (uint32_t i0 = 0; i0 < v.nv && v.v_key[i0] < best - slack; i0 += RG) {
+    for (uint32_t i0 = 0; i0 < v.nv; i0 += RG) {
+        if (!(v.v_key[i0] < best - slack)) {
+            if (SAFE) m = fminf(m, __double2float_rd(v.v_key[i0] + slack));
+            break;
+        }
         const uint32_t i = i0 + gl;
         double val = inf;
-        if (i < v.nv && v.v_key[i] < best - slack) {
+        if (i < v.nv && !(v.v_key[i] < best - slack)) {
+            if (SAFE) m = fminf(m, __double2float_rd(v.v_key[i] + slack));
+        } else if (i < v.nv) {
             const double4 p = v.v_p[i];
             const double d2 = sq3(x, y, z, p.x, p.y, p.z);
             if (sqrt_lt(d2, best)) val = sqrt(d2);
+            else if (SAFE) m = fminf(m, x_sqrt_below(d2));
         }
+        const float own = __double2float_rd(val);
         int w = int(i);
         x_argmin<RG>(gm, val, w);
+        if (SAFE && (!(val < best) || w != int(i))) m = fminf(m, own);
         if (val < best) {
+            if (SAFE) m = fminf(m, __double2float_rd(best));
+            safe.pos = uint32_t(w);
             const double4 p = v.v_p[w];
             best = val, e.kind = XF_VERTEX, e.id = v.v_id[w], e.qx = p.x, e.qy = p.y, e.qz = p.z;
         }
     }
     e.value = probe - best;
+    safe.kind = e.kind;
+    if (SAFE && e.kind != XF_BEYOND) {
+        safe.r = x_safe_radius(blocked, m, best);
+#pragma unroll
+        for (int o = RG / 2; o; o >>= 1) safe.r = fminf(safe.r, __shfl_xor_sync(gm, safe.r, o));
+    }
     return e;
 }
 
@@ -926,24 +1099,42 @@ __device__ __forceinline__ void x_edge(const XView& v, const DArr& A, const DLat
     XEval last;
     double t0 = 0.0, g0 = fa, t1 = 1.0, g1 = fb;
     int side = 0;
-    bool converged = false;
     uint32_t evals = 0;
     const bool spheres = A.flags & DARR_SPHERES;
-    auto eval = [&](double x, double y, double z) {
-        if (spheres)
-            return RG == 1 ? x_eval_spheres<COUNT>(v, band, x, y, z, ops) : x_eval_spheres_group<RG>(v, band, x, y, z, gl, gm);
-        return RG == 1 ? x_eval<COUNT>(v, A.circ, probe, band, x, y, z, ops)
-                       : x_eval_group<RG>(v, A.circ, probe, band, x, y, z, gl, gm);
+    const double edge = sqrt(dx * dx + dy * dy + dz * dz);
+    // SAFE: the first point is walked; the next ones lie close to it (the surface
+    // is nearly flat over an edge), mostly within the radius its winner is
+    // certain in, and then take one candidate instead of the lists.
+    constexpr bool SAFE = !COUNT && RG != 8;
+    XSafe safe;
+    safe.r = 0.0f;
+    double t_safe = 0.0;
+    auto eval = [&](double x, double y, double z, XEval& e) {
+        if (spheres) {
+            e = RG == 1 ? x_eval_spheres<COUNT>(v, band, x, y, z, ops) : x_eval_spheres_group<RG>(v, band, x, y, z, gl, gm);
+            return;
+        }
+        if (SAFE && float(fabs(t - t_safe) * edge) * 1.0001f + 1e-9f < safe.r &&
+            x_eval_again<RG>(v, A.circ, probe, band, x, y, z, safe, e, gl, gm))
+            return;
+        t_safe = t;
+        e = RG == 1 ? x_eval<COUNT, SAFE>(v, A.circ, probe, band, x, y, z, safe, ops)
+                    : x_eval_group<RG, SAFE>(v, A.circ, probe, band, x, y, z, safe, gl, gm);
     };
-    for (int it = 0; it < X_MAX_ITER; it++) {
+    // Up to X_MAX_ITER Newton or Illinois steps, then bisection.
+    for (int it = 0; it < X_MAX_ITER + X_MAX_BISECT; it++) {
+        const bool bisect = it >= X_MAX_ITER;
+        if (bisect) t = 0.5 * (t0 + t1);
         const double x = pax + dx * t, y = pay + dy * t, z = paz + dz * t;
-        const XEval e = eval(x, y, z);
+        eval(x, y, z, last);
         evals++;
-        last = e;
-        const double g = e.value;
-        if (fabs(g) <= X_TOL) {
-            converged = true;
-            break;
+        const double g = last.value;
+        if (fabs(g) <= X_TOL) break;
+        if (bisect) {
+            if ((t1 - t0) * edge <= 2.0 * X_TOL) break;
+            if ((g < 0.0) == (g0 < 0.0)) t0 = t;
+            else t1 = t;
+            continue;
         }
         if ((g < 0.0) == (g0 < 0.0)) {
             t0 = t, g0 = g;
@@ -955,34 +1146,20 @@ __device__ __forceinline__ void x_edge(const XView& v, const DArr& A, const DLat
             side = 1;
         }
         double slope = 0.0;
-        if (e.kind != XF_SOLVENT && e.kind != XF_BEYOND) {
+        if (last.kind != XF_SOLVENT && last.kind != XF_BEYOND) {
             // gradient (extract.rs:539-549): towards the closest point (SES)
             // or away from the sphere's centre (a sphere field).
-            const double wx = spheres ? x - e.qx : e.qx - x, wy = spheres ? y - e.qy : e.qy - y,
-                         wz = spheres ? z - e.qz : e.qz - z;
+            const double wx = spheres ? x - last.qx : last.qx - x, wy = spheres ? y - last.qy : last.qy - y,
+                         wz = spheres ? z - last.qz : last.qz - z;
             const double len = sqrt(wx * wx + wy * wy + wz * wz);
             if (len > 1e-12) slope = (wx / len) * dx + (wy / len) * dy + (wz / len) * dz;
         }
         const double newton = t - g / slope;
-        if (fabs(slope) > 1e-3 * sqrt(dx * dx + dy * dy + dz * dz) && newton > t0 && newton < t1) {
+        if (fabs(slope) > 1e-3 * edge && newton > t0 && newton < t1) {
             t = newton;
         } else {
             const double s = (t0 * g1 - t1 * g0) / (g1 - g0);
             t = (isfinite(s) && s > t0 && s < t1) ? s : 0.5 * (t0 + t1);
-        }
-    }
-    if (!converged) {
-        const double len = sqrt(dx * dx + dy * dy + dz * dz);
-        const bool neg0 = g0 < 0.0;
-        for (int it = 0; it < X_MAX_BISECT; it++) {
-            t = 0.5 * (t0 + t1);
-            const double x = pax + dx * t, y = pay + dy * t, z = paz + dz * t;
-            const XEval e = eval(x, y, z);
-            evals++;
-            last = e;
-            if (fabs(e.value) <= X_TOL || (t1 - t0) * len <= 2.0 * X_TOL) break;
-            if ((e.value < 0.0) == neg0) t0 = t;
-            else t1 = t;
         }
     }
     if (gl) return;
