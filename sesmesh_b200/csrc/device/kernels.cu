@@ -415,15 +415,26 @@ __device__ __forceinline__ unsigned warp_inclusive_scan(unsigned v) {
 // One warp: the lists of work item `item` (a sampled sub-block).
 // WIDE: blocker rows through near_members (four lookups in flight), which
 // pays where a sub-block's lists fill several rounds of the warp's lanes
-// (a 2.4 M-sphere shell at 1 A, 141 near spheres per sub-block: 291 -> 256
-// ms; a 58,800-sphere assembly at 0.25 A, 30: 12.1 -> 13.2 ms); otherwise a
-// lane walks its row one lookup at a time.
-template <bool MANY, bool WIDE>
+// (by warps, a 2.4 M-sphere shell at 1 A, 141 near spheres per sub-block: 291
+// -> 256 ms; a 58,800-sphere assembly at 0.25 A, 30: 12.1 -> 13.2 ms);
+// otherwise a lane walks its row one lookup at a time.
+// TEAM: warps that share the item (1, or the block's).  The scans, whose order
+// decides the lists', are a warp each and run side by side; the sorts, the
+// blocker rows and the writes go over all lanes.
+template <bool MANY, bool WIDE, int TEAM>
 __device__ __forceinline__ void gather_item(uint32_t item, const DArr& A0, const DLat& L0, const int4* keys,
                                             const uint32_t* work, const GatherOut& O, const GatherCaps& caps,
                                             const Scene& S, unsigned char* smem_raw) {
+    constexpr int NT = 32 * TEAM;
+    __shared__ unsigned long long share[TEAM > 1 ? 8 : 1];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    unsigned char* base = smem_raw + size_t(wib) * gather_smem_bytes(caps);
+    const int tid = TEAM == 1 ? lane : int(threadIdx.x), wt = TEAM == 1 ? 0 : wib;
+    auto sync = [] {
+        if (TEAM == 1) __syncwarp();
+        else __syncthreads();
+    };
+    if (TEAM > 1) sync();  // the previous item's lists are no longer read
+    unsigned char* base = smem_raw + (TEAM == 1 ? size_t(wib) * gather_smem_bytes(caps) : 0);
     double* s_key = reinterpret_cast<double*>(base);
     double* c_key = s_key + caps.s;
     uint32_t* near_ids = reinterpret_cast<uint32_t*>(c_key + caps.c);
@@ -470,9 +481,9 @@ __device__ __forceinline__ void gather_item(uint32_t item, const DArr& A0, const
     const double r_circ = win ? reach_x + A.rho_max : reach + A.rho_max, r_vert = win ? reach_x : reach;
     bool differ = false;
 
-    if (lane == 0) rec[R_FLAGS] = 0;
+    if (tid == 0) rec[R_FLAGS] = 0;
     auto overflow = [&](uint32_t bit) {
-        if (lane == 0) {
+        if (tid == 0) {
             rec[R_FLAGS] |= bit;
             unsigned long long q = atomicAdd(&O.counters[bit == REC_OVERFLOW ? CNT_OVERFLOW : CNT_NOMEM], 1ull);
             if (bit == REC_OVERFLOW && O.retry) O.retry[q] = j;
@@ -490,8 +501,8 @@ __device__ __forceinline__ void gather_item(uint32_t item, const DArr& A0, const
     // below (its rounded distance exceeds each of them), so it is neither
     // kept nor a disagreement, and its square root is not taken.
     uint32_t* scan_buf = reinterpret_cast<uint32_t*>(near_tab);
-    int nn = 0;
-    warp_scan_box(A.gs, bx, by, bz, r_sph, lane, [&](bool valid, uint32_t k) {
+    int nn = 0, n_in = 0, ns = 0, nc = 0, nv = 0;
+    if (wt == 0) warp_scan_box(A.gs, bx, by, bz, r_sph, lane, [&](bool valid, uint32_t k) {
         bool keep = false, contains = false;
         if (valid && A.status[k] != STATUS_CONTAINED) {
             double4 c = A.sph[k];
@@ -513,15 +524,14 @@ __device__ __forceinline__ void gather_item(uint32_t item, const DArr& A0, const
         int pos = warp_append(keep, nn);
         if (pos >= 0 && pos < caps.near) scan_buf[pos] = k | (contains ? 0x80000000u : 0u);
     });
-    if (lane == 0) atomicMax(&O.counters[CNT_MAXNN], (unsigned long long)nn);
-    if (nn > caps.near) return overflow(REC_OVERFLOW);
+    if (wt == 0 && lane == 0) atomicMax(&O.counters[CNT_MAXNN], (unsigned long long)nn);
+    if (TEAM == 1 && nn > caps.near) return overflow(REC_OVERFLOW);
     __syncwarp();
-    int n_in = 0;
-    for (int b0 = 0; b0 < nn; b0 += 32) {
-        const int i = b0 + lane;
-        n_in += __popc(__ballot_sync(0xffffffffu, i < nn && (scan_buf[i] >> 31)));
-    }
-    {
+    if (wt == 0 && nn <= caps.near) {
+        for (int b0 = 0; b0 < nn; b0 += 32) {
+            const int i = b0 + lane;
+            n_in += __popc(__ballot_sync(0xffffffffu, i < nn && (scan_buf[i] >> 31)));
+        }
         const uint32_t below = (1u << lane) - 1u;
         int at_in = 0, at_out = n_in;
         for (int b0 = 0; b0 < nn; b0 += 32) {
@@ -533,39 +543,27 @@ __device__ __forceinline__ void gather_item(uint32_t item, const DArr& A0, const
             if (g) near_ids[at_out + __popc(mg & below)] = w;
             at_in += __popc(mf), at_out += __popc(mg);
         }
-    }
-    __syncwarp();
-    // The near table for blocker lookups (positions in the near list).
-    for (uint32_t i = lane; i < (1u << tab_bits); i += 32) near_tab[i] = 0xFFFFu;
-    __syncwarp();
-    for (int i = lane; i < nn; i += 32) {
-        const uint32_t mask = (1u << tab_bits) - 1;
-        uint32_t h = near_hash(near_ids[i], tab_bits);
-        while (atomicCAS(&near_tab[h], (unsigned short)0xFFFFu, (unsigned short)i) != (unsigned short)0xFFFFu)
-            h = (h + 1) & mask;  // ends: at most half of the slots are taken
-    }
-    __syncwarp();
-    // Class S candidates among the near spheres.
-    int ns = 0;
-    for (int b0 = 0; b0 < nn; b0 += 32) {
-        int i = b0 + lane;
-        bool p = false;
-        double lb = 0;
-        uint32_t k = 0;
-        if (i < nn && !spheres) {
-            k = near_ids[i];
-            if (A.status[k] == STATUS_EXPOSED) {
-                double4 c = A.sph[k];
-                lb = fabs(dist3(bx, by, bz, c.x, c.y, c.z) - c.w);
-                p = lb <= reach;
+        __syncwarp();
+        // Class S candidates among the near spheres.
+        for (int b0 = 0; b0 < nn; b0 += 32) {
+            int i = b0 + lane;
+            bool p = false;
+            double lb = 0;
+            uint32_t k = 0;
+            if (i < nn && !spheres) {
+                k = near_ids[i];
+                if (A.status[k] == STATUS_EXPOSED) {
+                    double4 c = A.sph[k];
+                    lb = fabs(dist3(bx, by, bz, c.x, c.y, c.z) - c.w);
+                    p = lb <= reach;
+                }
             }
+            int pos = warp_append(p, ns);
+            if (pos >= 0 && pos < caps.s) s_key[pos] = lb, s_id[pos] = k, s_loc[pos] = uint32_t(i);
         }
-        int pos = warp_append(p, ns);
-        if (pos >= 0 && pos < caps.s) s_key[pos] = lb, s_id[pos] = k, s_loc[pos] = uint32_t(i);
     }
     // Class C candidates.
-    int nc = 0;
-    warp_scan_box(A.gc, bx, by, bz, r_circ, lane, [&](bool valid, uint32_t ci) {
+    if (wt == (TEAM > 1 ? 1 : 0)) warp_scan_box(A.gc, bx, by, bz, r_circ, lane, [&](bool valid, uint32_t ci) {
         double d = valid ? circle_reach_dist_above(A, bx, by, bz, ci, win ? reach_x : reach) : 0.0;
         bool p = valid && d <= reach;
         if (win && valid) differ |= (d <= reach_x) != p;
@@ -573,8 +571,7 @@ __device__ __forceinline__ void gather_item(uint32_t item, const DArr& A0, const
         if (pos >= 0 && pos < caps.c) c_key[pos] = d, c_id[pos] = ci;
     });
     // Class V, cell-scan order.
-    int nv = 0;
-    warp_scan_box(A.gv, bx, by, bz, r_vert, lane, [&](bool valid, uint32_t vi) {
+    if (wt == (TEAM > 2 ? 2 : 0)) warp_scan_box(A.gv, bx, by, bz, r_vert, lane, [&](bool valid, uint32_t vi) {
         bool p = false;
         if (valid) {
             double4 q = A.vert[vi];
@@ -585,69 +582,100 @@ __device__ __forceinline__ void gather_item(uint32_t item, const DArr& A0, const
         int pos = warp_append(p, nv);
         if (pos >= 0 && pos < caps.v) v_id[pos] = vi;
     });
-    if (lane == 0) {
+    if constexpr (TEAM > 1) {
+        if (lane == 0) {
+            if (wt == 0) share[0] = nn, share[1] = n_in, share[2] = ns;
+            if (wt == 1) share[3] = nc;
+            if (wt == 2) share[4] = nv;
+        }
+        __syncthreads();
+        nn = int(share[0]), n_in = int(share[1]), ns = int(share[2]), nc = int(share[3]), nv = int(share[4]);
+        if (nn > caps.near) return overflow(REC_OVERFLOW);
+    }
+    if (tid == 0) {
         atomicMax(&O.counters[CNT_MAXNS], (unsigned long long)ns);
         atomicMax(&O.counters[CNT_MAXNC], (unsigned long long)nc);
         atomicMax(&O.counters[CNT_MAXNV], (unsigned long long)nv);
     }
     if (ns > caps.s || nc > caps.c || nv > caps.v) return overflow(REC_OVERFLOW);
-    __syncwarp();
+    sync();
+    // The near table for blocker lookups (positions in the near list).
+    for (uint32_t i = tid; i < (1u << tab_bits); i += NT) near_tab[i] = 0xFFFFu;
+    sync();
+    for (int i = tid; i < nn; i += NT) {
+        const uint32_t mask = (1u << tab_bits) - 1;
+        uint32_t h = near_hash(near_ids[i], tab_bits);
+        while (atomicCAS(&near_tab[h], (unsigned short)0xFFFFu, (unsigned short)i) != (unsigned short)0xFFFFu)
+            h = (h + 1) & mask;  // ends: at most half of the slots are taken
+    }
     // Rank sorts: (key, index) pairs are distinct, so ranks are a permutation.
-    for (int i = lane; i < ns; i += 32) {
+    for (int i = tid; i < ns; i += NT) {
         double kv = s_key[i];
         uint32_t id = s_id[i];
         int rank = 0;
         for (int q = 0; q < ns; q++) rank += (s_key[q] < kv) || (s_key[q] == kv && s_id[q] < id);
         s_perm[rank] = uint32_t(i);
     }
-    for (int i = lane; i < nc; i += 32) {
+    for (int i = tid; i < nc; i += NT) {
         double kv = c_key[i];
         uint32_t id = c_id[i];
         int rank = 0;
         for (int q = 0; q < nc; q++) rank += (c_key[q] < kv) || (c_key[q] == kv && c_id[q] < id);
         c_perm[rank] = uint32_t(i);
     }
-    __syncwarp();
-    // Blocker counts and offsets, in sorted order.
-    unsigned run = 0;
-    if (lane == 0) s_off[0] = 0;
-    for (int b0 = 0; b0 < ns; b0 += 32) {
-        int r = b0 + lane;
-        unsigned cnt = 0;
-        if (r < ns) {
-            uint32_t k = s_id[s_perm[r]];
-            if constexpr (WIDE)
-                cnt = near_members(near_tab, tab_bits, near_ids, A.nb_items, A.nb_off[k], A.nb_off[k + 1], nullptr,
-                                   nullptr);
-            else
-                for (uint32_t p = A.nb_off[k], e = A.nb_off[k + 1]; p < e; p++)
-                    cnt += lookup_near(near_tab, tab_bits, near_ids, A.nb_items[p]) >= 0;
+    sync();
+    // Blocker counts and offsets, in sorted order.  Rows are cut into up to
+    // eight parts while a part per lane leaves lanes free (a lane walks 50 to
+    // 70 neighbours of a sphere, and a sub-block at 0.25 A has a dozen such
+    // rows: 58,800 spheres 14.5 -> 11.8 ms); a lane keeps its part's offset
+    // for the writes.
+    auto split = [](int n) {
+        int g = 0;
+        while (g < 3 && (n << (g + 1)) <= NT) g++;
+        return g;
+    };
+    auto part_of = [&](const uint32_t* off, uint32_t k, int part, int g, uint32_t& a, uint32_t& e) {
+        const uint32_t p0 = off[k], len = off[k + 1] - p0, q = uint32_t(part & ((1 << g) - 1));
+        a = p0 + ((len * q) >> g), e = p0 + ((len * (q + 1)) >> g);
+    };
+    auto count_rows = [&](int n, int g, const uint32_t* perm, const uint32_t* id, const uint32_t* row,
+                          const uint32_t* items, uint32_t* off, uint32_t& mine) {
+        unsigned run = 0;
+        if (tid == 0) off[0] = 0;
+        for (int b0 = 0; b0 < (n << g); b0 += NT) {
+            const int part = b0 + tid, r = part >> g;
+            unsigned cnt = 0;
+            if (r < n) {
+                uint32_t a, e;
+                part_of(row, id[perm[r]], part, g, a, e);
+                if constexpr (WIDE)
+                    cnt = near_members(near_tab, tab_bits, near_ids, items, a, e, nullptr, nullptr);
+                else
+                    for (uint32_t p = a; p < e; p++) cnt += lookup_near(near_tab, tab_bits, near_ids, items[p]) >= 0;
+            }
+            unsigned inc = warp_inclusive_scan(cnt);
+            unsigned all = __shfl_sync(0xffffffffu, inc, 31);
+            if constexpr (TEAM > 1) {
+                if (lane == 31) share[wt] = inc;
+                __syncthreads();
+                all = 0;
+                for (int w = 0; w < TEAM; w++) {
+                    if (w == wt) inc += all;
+                    all += unsigned(share[w]);
+                }
+                __syncthreads();
+            }
+            if (b0 == 0) mine = inc - cnt;
+            if (r < n && (part & ((1 << g) - 1)) == (1 << g) - 1) off[r + 1] = run + inc;
+            run += all;
         }
-        unsigned inc = warp_inclusive_scan(cnt);
-        if (r < ns) s_off[r + 1] = run + inc;
-        run += __shfl_sync(0xffffffffu, inc, 31);
-    }
-    const unsigned nsb = run;
-    run = 0;
-    if (lane == 0) c_off[0] = 0;
-    for (int b0 = 0; b0 < nc; b0 += 32) {
-        int r = b0 + lane;
-        unsigned cnt = 0;
-        if (r < nc) {
-            uint32_t ci = c_id[c_perm[r]];
-            if constexpr (WIDE)
-                cnt = near_members(near_tab, tab_bits, near_ids, A.cb_items, A.cb_off[ci], A.cb_off[ci + 1], nullptr,
-                                   nullptr);
-            else
-                for (uint32_t p = A.cb_off[ci], e = A.cb_off[ci + 1]; p < e; p++)
-                    cnt += lookup_near(near_tab, tab_bits, near_ids, A.cb_items[p]) >= 0;
-        }
-        unsigned inc = warp_inclusive_scan(cnt);
-        if (r < nc) c_off[r + 1] = run + inc;
-        run += __shfl_sync(0xffffffffu, inc, 31);
-    }
-    const unsigned ncb = run;
-    __syncwarp();
+        return run;
+    };
+    const int s_split = split(ns), c_split = split(nc);
+    uint32_t s_mine = 0, c_mine = 0;
+    const unsigned nsb = count_rows(ns, s_split, s_perm, s_id, A.nb_off, A.nb_items, s_off, s_mine);
+    const unsigned ncb = count_rows(nc, c_split, c_perm, c_id, A.cb_off, A.cb_items, c_off, c_mine);
+    sync();
 
     // Space: ids (CSR words) and the packed f32 block the sampler stages.
     const unsigned long long ids_words =
@@ -655,13 +683,19 @@ __device__ __forceinline__ void gather_item(uint32_t item, const DArr& A0, const
     const unsigned long long tail_words = 2ull * ns + 1 + nsb + 2ull * nc + 1 + ncb;
     const unsigned long long units = 2ull * nn + ns + 3ull * nc + nv + (tail_words + 3) / 4;
     unsigned long long ids_base = 0, pack_base = 0;
-    if (lane == 0) {
+    if (tid == 0) {
         ids_base = atomicAdd(&O.counters[CNT_IDS], ids_words);
         pack_base = atomicAdd(&O.counters[CNT_PACK], units);
         atomicMax(&O.counters[CNT_MAXPACK], units);
     }
-    ids_base = __shfl_sync(0xffffffffu, ids_base, 0);
-    pack_base = __shfl_sync(0xffffffffu, pack_base, 0);
+    if constexpr (TEAM > 1) {
+        if (tid == 0) share[6] = ids_base, share[7] = pack_base;
+        __syncthreads();
+        ids_base = share[6], pack_base = share[7];
+    } else {
+        ids_base = __shfl_sync(0xffffffffu, ids_base, 0);
+        pack_base = __shfl_sync(0xffffffffu, pack_base, 0);
+    }
     if (ids_base + ids_words > O.ids_cap || pack_base + units > O.pack_cap || units > O.unit_cap)
         return overflow(REC_NOMEM);
 
@@ -691,7 +725,23 @@ __device__ __forceinline__ void gather_item(uint32_t item, const DArr& A0, const
     uint32_t* p_coff = p_sblk + nsb;
     uint32_t* p_cblk = p_coff + nc + 1;
 
-    for (int i = lane; i < nn; i += 32) {
+    auto write_rows = [&](int n, int g, const uint32_t* perm, const uint32_t* id, const uint32_t* row,
+                          const uint32_t* items, const uint32_t* off, uint32_t mine, uint32_t* w, uint32_t* pk) {
+        for (int part = tid; part < (n << g); part += NT) {
+            const int r = part >> g;
+            uint32_t a, e, o = g ? mine : off[r];
+            part_of(row, id[perm[r]], part, g, a, e);
+            if constexpr (WIDE) {
+                near_members(near_tab, tab_bits, near_ids, items, a, e, w + o, pk + o);
+            } else {
+                for (uint32_t p = a; p < e; p++) {
+                    int l = lookup_near(near_tab, tab_bits, near_ids, items[p]);
+                    if (l >= 0) w[o] = uint32_t(l), pk[o] = uint32_t(l), o++;
+                }
+            }
+        }
+    };
+    for (int i = tid; i < nn; i += NT) {
         uint32_t k = near_ids[i];
         w_near[i] = k;
         double4 c = A.sph[k];
@@ -702,59 +752,41 @@ __device__ __forceinline__ void gather_item(uint32_t item, const DArr& A0, const
         // A sphere field has no blockers: its samples take R itself.
         p_nearT[i] = make_float4(x, y, z, spheres ? r32 : rt * rt);
     }
-    for (int r = lane; r <= ns; r += 32) w_soff[r] = s_off[r], p_soff[r] = s_off[r];
+    for (int r = tid; r <= ns; r += NT) w_soff[r] = s_off[r], p_soff[r] = s_off[r];
     // Pruning keys: every sample the sub-block evaluates lies within rho of
     // its centre, and |d - R| and the circle distance are 1-Lipschitz, so a
     // candidate whose centre value minus rho exceeds the sample's current best
     // cannot improve it; PRUNE_MARGIN (1e-3 A) covers f32 rounding, so the
     // skipped candidates are exactly those whose test would fail.
-    for (int r = lane; r < ns; r += 32)
+    for (int r = tid; r < ns; r += NT)
         p_skey[r] = __double2float_rd(s_key[s_perm[r]] - rho - PRUNE_MARGIN);
-    for (int r = lane; r < nc; r += 32)
+    for (int r = tid; r < nc; r += NT)
         p_ckey[r] = __double2float_rd(c_key[c_perm[r]] - rho - PRUNE_MARGIN);
-    for (int r = lane; r < ns; r += 32) {
+    for (int r = tid; r < ns; r += NT) {
         uint32_t i = s_perm[r], k = s_id[i];
         w_s[r] = k;
         double4 c = A.sph[k];
         p_s[r] = make_float4(float(c.x - L.fx), float(c.y - L.fy), float(c.z - L.fz), float(c.w));
-        uint32_t o = s_off[r];
-        if constexpr (WIDE) {
-            near_members(near_tab, tab_bits, near_ids, A.nb_items, A.nb_off[k], A.nb_off[k + 1], w_sblk + o,
-                         p_sblk + o);
-        } else {
-            for (uint32_t p = A.nb_off[k], e = A.nb_off[k + 1]; p < e; p++) {
-                int l = lookup_near(near_tab, tab_bits, near_ids, A.nb_items[p]);
-                if (l >= 0) w_sblk[o] = uint32_t(l), p_sblk[o] = uint32_t(l), o++;
-            }
-        }
     }
-    for (int r = lane; r <= nc; r += 32) w_coff[r] = c_off[r], p_coff[r] = c_off[r];
-    for (int r = lane; r < nc; r += 32) {
+    write_rows(ns, s_split, s_perm, s_id, A.nb_off, A.nb_items, s_off, s_mine, w_sblk, p_sblk);
+    for (int r = tid; r <= nc; r += NT) w_coff[r] = c_off[r], p_coff[r] = c_off[r];
+    for (int r = tid; r < nc; r += NT) {
         uint32_t ci = c_id[c_perm[r]];
         w_c[r] = ci;
         const double* c = A.circ + 12 * size_t(ci);
         p_c[3 * r] = make_float4(float(c[0] - L.fx), float(c[1] - L.fy), float(c[2] - L.fz), float(c[9]));
         p_c[3 * r + 1] = make_float4(float(c[3]), float(c[4]), float(c[5]), float(c[6]));
         p_c[3 * r + 2] = make_float4(float(c[7]), float(c[8]), 0.0f, 0.0f);
-        uint32_t o = c_off[r];
-        if constexpr (WIDE) {
-            near_members(near_tab, tab_bits, near_ids, A.cb_items, A.cb_off[ci], A.cb_off[ci + 1], w_cblk + o,
-                         p_cblk + o);
-        } else {
-            for (uint32_t p = A.cb_off[ci], e = A.cb_off[ci + 1]; p < e; p++) {
-                int l = lookup_near(near_tab, tab_bits, near_ids, A.cb_items[p]);
-                if (l >= 0) w_cblk[o] = uint32_t(l), p_cblk[o] = uint32_t(l), o++;
-            }
-        }
     }
-    for (int i = lane; i < nv; i += 32) {
+    write_rows(nc, c_split, c_perm, c_id, A.cb_off, A.cb_items, c_off, c_mine, w_cblk, p_cblk);
+    for (int i = tid; i < nv; i += NT) {
         uint32_t vi = v_id[i];
         w_v[i] = vi;
         double4 q = A.vert[vi];
         p_v[i] = make_float4(float(q.x - L.fx), float(q.y - L.fy), float(q.z - L.fz), 0.0f);
     }
-    const bool any_differ = __any_sync(0xffffffffu, differ);
-    if (lane == 0) {
+    const bool any_differ = TEAM == 1 ? __any_sync(0xffffffffu, differ) : __syncthreads_or(differ);
+    if (tid == 0) {
         if (win) O.window[j] = any_differ ? 1 : 0;
         rec[R_IDS] = uint32_t(ids_base);
         rec[R_INSIDE] = uint32_t(n_in);
@@ -771,14 +803,26 @@ __device__ __forceinline__ void gather_item(uint32_t item, const DArr& A0, const
 
 // Warp per work item, the grid striding over the items (many structures:
 // the item count is read on the device).
-template <bool MANY, bool WIDE>
+template <bool MANY>
 __global__ void __launch_bounds__(256, MANY ? 2 : 4) k_gather(DArr A0, DLat L0, const int4* keys, const uint32_t* work, uint32_t n_work, GatherOut O,
                          GatherCaps caps, Scene S) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const uint32_t n = S.n_work ? uint32_t(*S.n_work) : n_work;
     const uint32_t wpb = blockDim.x >> 5;
     for (uint32_t item = blockIdx.x * wpb + (threadIdx.x >> 5); item < n; item += gridDim.x * wpb)
-        gather_item<MANY, WIDE>(item, A0, L0, keys, work, O, caps, S, smem_raw);
+        gather_item<MANY, false, 1>(item, A0, L0, keys, work, O, caps, S, smem_raw);
+}
+
+// A block of four warps per work item.
+constexpr int GATHER_TEAM = 4;
+template <bool WIDE>
+__global__ void __launch_bounds__(32 * GATHER_TEAM, 8) k_gather_team(DArr A0, DLat L0, const int4* keys,
+                                                                     const uint32_t* work, uint32_t n_work,
+                                                                     GatherOut O, GatherCaps caps, Scene S) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const uint32_t n = S.n_work ? uint32_t(*S.n_work) : n_work;
+    for (uint32_t item = blockIdx.x; item < n; item += gridDim.x)
+        gather_item<false, WIDE, GATHER_TEAM>(item, A0, L0, keys, work, O, caps, S, smem_raw);
 }
 
 // ---------------------------------------------------------------------------
@@ -2324,20 +2368,32 @@ void launch_substates(const DArr& A, const DLat& L, const int4* keys, uint32_t n
     else k_substates<false><<<n, 256, 0, s>>>(A, L, keys, n, rec, sampled, Scene{});
 }
 
+// A block of four warps per sub-block where the lists take several rounds of
+// a warp's lanes (the caps come from the largest lists seen) and a warp's
+// list scratch leaves an SM some ten warps: 2.4 M spheres at 1 A 264 -> 86
+// ms, 5,003 at 0.5 A (8,483 sub-blocks) 0.95 -> 0.65; and for a wave of warps
+// or less, which waits for one sub-block's chain: 331 spheres (1,400) 0.28 ->
+// 0.09.  For more sub-blocks with short lists the warps' scans are the work
+// and a warp each does best: 18,752 sub-blocks of 6.5 KB 0.58 against 0.87,
+// 398,291 of them 11.8 against 19.2 ms.
+constexpr uint32_t GATHER_TEAM_MAX = 148 * 32;
+
 cudaError_t launch_gather(const DArr& A, const DLat& L, const int4* keys, const uint32_t* work, uint32_t n,
                           const GatherOut& O, const GatherCaps& caps, int warps, cudaStream_t s, const Scene* many,
                           const unsigned long long* n_dev) {
     if (!n) return cudaSuccess;
     size_t smem = gather_smem_bytes(caps) * size_t(warps);
-    // Lists of several warp rounds (the caps come from the largest lists
-    // seen): blocker rows with four lookups in flight.
-    auto kern = many ? k_gather<true, false> : caps.near >= 128 ? k_gather<false, true> : k_gather<false, false>;
+    // Lists of several warp rounds: blocker rows with four lookups in flight.
+    const bool rounds = caps.near >= 128;
+    const bool team = !many && (rounds || n <= GATHER_TEAM_MAX);
+    if (team) smem = gather_smem_bytes(caps), warps = GATHER_TEAM;
+    auto kern = many ? k_gather<true> : !team ? k_gather<false> : rounds ? k_gather_team<true> : k_gather_team<false>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e != cudaSuccess) return e;
     COUNT(1);
     // Many structures: n is an upper bound of the device count; the grid
     // strides (a few waves of blocks, not one per possible item).
-    uint32_t blocks = (n + warps - 1) / warps;
+    uint32_t blocks = team ? n : (n + warps - 1) / warps;
     if (many) blocks = std::min<uint32_t>(blocks, 148u * 32u);
     Scene S{};
     if (many) S = *many;
