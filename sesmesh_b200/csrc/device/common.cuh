@@ -265,34 +265,60 @@ __device__ __forceinline__ double circle_reach_dist_above(const DArr& A, double 
     return sqrt(a2 + (wl - c[9]) * (wl - c[9]));
 }
 
-// SesField::ses_eval distance (field/point.rs:385-411), one warp.  The result
-// is min(cutoff, min over unblocked candidates), which does not depend on the
-// visiting order, so lanes keep partial minima that are merged at the end.
-// inside_known: 1 or 0 when the caller's scan already settled whether some
-// sphere contains the point (it covered every sphere that can), -1 to scan.
-__device__ inline double ses_eval_warp(const DArr& A, double x, double y, double z, double cutoff, int lane,
-                                       int inside_known = -1) {
-    bool inside = inside_known > 0;
-    if (inside_known < 0)
-        warp_for_near(A.gs, x, y, z, A.max_expanded, lane, [&](uint32_t k) {
-            if (!inside && A.status[k] != STATUS_CONTAINED) {
-                double4 c = A.sph[k];
-                if (sqrt_lt(sq3(x, y, z, c.x, c.y, c.z), c.w)) inside = true;
-            }
+// uniform_sign's answer from SesField::ses_eval (field/point.rs:385-411), one
+// warp: with m the least value of the unblocked candidates (at most cutoff),
+// 1 where fl(probe - m) > margin, 0 where it is < -margin, else -1.  Only the
+// answer is wanted: one unblocked candidate in the band between leaves the
+// candidates that could still turn it to 1, those below probe - margin (none
+// when that is not above 0), so each lane's limit drops to that, and the
+// warp's between the classes.  The vertices come first: they have no
+// blockers, and some lie within the band of most points near the surface.
+// 58,800 spheres at 0.25 A: sub-block states 7.53 -> 5.43 ms, classification
+// 2.15 -> 1.02; 2.4 M at 1 A 15.7 -> 2.9 and 6.9 -> 1.35.
+__device__ inline int ses_sign_warp(const DArr& A, double x, double y, double z, double margin, double cutoff,
+                                    int lane) {
+    const double probe = A.probe;
+    // Values from here on cannot answer 1 (1e-9 is far above the rounding).
+    const double low = fmax(probe - margin + 1e-9, 0.0);
+    bool out = false, mid = !(probe - cutoff < -margin);
+    double best = mid ? fmin(cutoff, low) : cutoff;
+    auto found = [&](double v) {  // an unblocked candidate's value, below best
+        if (probe - v > margin) out = true, best = 0.0;
+        else if (!(probe - v < -margin)) mid = true, best = fmin(v, low);
+        else best = v;
+    };
+    // Merges the lanes' findings; true when the answer is settled.
+    auto settled = [&] {
+        out = __any_sync(0xffffffffu, out), mid = __any_sync(0xffffffffu, mid);
+        best = out ? 0.0 : mid ? fmin(best, low) : best;
+        best = warp_min(best);
+        return !(best > 0.0);
+    };
+    bool done = settled();
+    if (!done) {
+        warp_for_near(A.gv, x, y, z, best, lane, [&](uint32_t vi) {
+            const double4 p = A.vert[vi];
+            const double d2 = sq3(x, y, z, p.x, p.y, p.z);
+            if (sqrt_lt(d2, best)) found(sqrt(d2));
         });
-    if (!__any_sync(0xffffffffu, inside)) return 0.0;
-    double best = cutoff;
-    warp_for_near(A.gs, x, y, z, cutoff + A.max_expanded, lane, [&](uint32_t i) {
-        if (A.status[i] == STATUS_EXPOSED) best = try_sphere(A, x, y, z, i, best);
-    });
-    best = warp_min(best);
-    warp_for_near(A.gc, x, y, z, cutoff + A.rho_max, lane, [&](uint32_t ci) { best = try_circle(A, x, y, z, ci, best); });
-    warp_for_near(A.gv, x, y, z, cutoff, lane, [&](uint32_t vi) {
-        double4 p = A.vert[vi];
-        const double d2 = sq3(x, y, z, p.x, p.y, p.z);
-        if (sqrt_lt(d2, best)) best = sqrt(d2);
-    });
-    return warp_min(best);
+        done = settled();
+    }
+    if (!done) {
+        warp_for_near(A.gs, x, y, z, best + A.max_expanded, lane, [&](uint32_t i) {
+            if (A.status[i] != STATUS_EXPOSED) return;
+            const double v = try_sphere(A, x, y, z, i, best);
+            if (v < best) found(v);
+        });
+        done = settled();
+    }
+    if (!done) {
+        warp_for_near(A.gc, x, y, z, best + A.rho_max, lane, [&](uint32_t ci) {
+            const double v = try_circle(A, x, y, z, ci, best);
+            if (v < best) found(v);
+        });
+        settled();
+    }
+    return out ? 1 : mid ? -1 : 0;
 }
 
 // lattice::uniform_sign (field/lattice.rs:190-227), one warp: 1 uniformly
@@ -326,10 +352,8 @@ __device__ inline int uniform_sign_warp(const DArr& A, double x, double y, doubl
     if (s_sas >= margin) return 1;
     if (s_vdw <= -margin) return 0;
     double cutoff = A.probe + margin + CLASSIFY_EPS;
-    double v = A.probe - ses_eval_warp(A, x, y, z, cutoff, lane, __any_sync(0xffffffffu, inside) ? 1 : 0);
-    if (v > margin) return 1;
-    if (v < -margin) return 0;
-    return -1;
+    if (!__any_sync(0xffffffffu, inside)) return A.probe > margin ? 1 : -1;  // the value is probe
+    return ses_sign_warp(A, x, y, z, margin, cutoff, lane);
 }
 
 }  // namespace smb
