@@ -2156,6 +2156,11 @@ constexpr int REFINE_WARPS = 4;
 // refinement (ten or more blocks to an SM; at most 80 registers, so twelve
 // blocks where the regions allow).
 constexpr size_t PAIR_REGION_MAX = 20480;
+// Staging region of the eight-warp blocks for longer lists: four blocks, 32
+// warps, to an SM.  2.4 M spheres at 1 A (42 KB lists), refinement in ms: two
+// warps and 28 KB 200, four warps and 28 KB 196, eight warps and 55 KB 179
+// (most sub-blocks then need no second pass).
+constexpr size_t LIST_REGION = 55 * 1024;
 constexpr size_t MANY_REGION = 14 * 1024;  // and of the many-structure pass's
 
 struct RefinePlan {
@@ -2165,7 +2170,7 @@ struct RefinePlan {
 // OVF: a block-wide pass (WIDE) that lists the sub-blocks over its region
 // (the split pass); per-warp passes always can.
 template <int MODE, bool WIDE, bool MANY, int RG, int NT = 32 * REFINE_WARPS, bool COUNT = false, bool OVF = false>
-__global__ void __launch_bounds__(NT, NT == 64 ? 12 : (NT > 32 * REFINE_WARPS ? 2 : 1)) k_refine(
+__global__ void __launch_bounds__(NT, NT == 64 ? 12 : (NT > 256 ? 2 : OVF ? 4 : 1)) k_refine(
     DArr A0, DLat L0, RefineConsts RC0, const int4* keys, const uint32_t* work, const uint32_t* rec, const uint32_t* ids,
     const uint32_t* edges, const float2* edge_vals, const uint32_t* item_off, const uint32_t* item_edges,
     uint32_t n_host, RefOut out, const float2* start, RefinePlan P, unsigned long long* counters, Scene S,
@@ -2523,16 +2528,15 @@ cudaError_t launch_refine(const DArr& A, const DLat& L, const RefineConsts& RC, 
     P.cand_bytes = uint32_t(al(cand_bytes));
     const size_t narrow = size_t(REFINE_WARPS) * P.cand_bytes;
     const size_t wide = P.cand_bytes;
-    // Blocks of two warps that share one staging region per sub-block: of the
-    // largest sub-block's size where that is at most PAIR_REGION_MAX, else of
-    // the size asked for (default: an eighth of the SM's shared memory),
-    // handing the sub-blocks that outgrow it to a whole-block pass over a
-    // list.  The counting pass (and a caller without ovf): one region per
+    // Blocks that share one staging region per sub-block: two warps and the
+    // largest sub-block's size where that is at most PAIR_REGION_MAX, else
+    // eight warps and up to LIST_REGION (or the size asked for), handing the
+    // sub-blocks that outgrow it to a whole-block pass over a list.  The counting pass (and a caller without ovf): one region per
     // warp while four fit in a block, else one per block.
     const bool use_wide = narrow > smem_limit;
-    size_t small = region ? region / 128 * 128 : (smem_limit / 2 - 1024) / REFINE_WARPS / 128 * 128;
+    size_t small = region ? region / 128 * 128 : LIST_REGION;
     small = std::max<size_t>(std::min(small, size_t(P.cand_bytes)), 128);
-    const bool split = ovf && (use_wide || small < P.cand_bytes);
+    const bool split = ovf && (use_wide || small < P.cand_bytes || (!region && P.cand_bytes > PAIR_REGION_MAX));
     const size_t smem = use_wide ? wide : narrow;
     if (smem_out) *smem_out = smem;
     if (!n_items) return cudaSuccess;
@@ -2606,14 +2610,13 @@ cudaError_t launch_refine(const DArr& A, const DLat& L, const RefineConsts& RC, 
                               : k_refine<REFINE_WARM, true, false, 8, 32 * WIDE_LIST_WARPS>)
                        : (g32 ? k_refine<REFINE_PLAIN, true, false, 32, 32 * WIDE_LIST_WARPS>
                               : k_refine<REFINE_PLAIN, true, false, 8, 32 * WIDE_LIST_WARPS>);
-        // Two-warp blocks sharing a region of the same size over the
-        // sub-blocks that fit it (twice the warps per SM of per-warp regions).
-        auto kp = warm ? (g32 ? k_refine<REFINE_WARM, true, false, 32, 64, false, true>
-                              : k_refine<REFINE_WARM, true, false, 8, 64, false, true>)
-                       : (g32 ? k_refine<REFINE_PLAIN, true, false, 32, 64, false, true>
-                              : k_refine<REFINE_PLAIN, true, false, 8, 64, false, true>);
-        e = run(kp, PS, small, ovf, nullptr, n_items, 64);
-        if (e != cudaSuccess) return e;
+        // Eight-warp blocks over the sub-blocks that fit the region.
+        auto kp = warm ? (g32 ? k_refine<REFINE_WARM, true, false, 32, 256, false, true>
+                              : k_refine<REFINE_WARM, true, false, 8, 256, false, true>)
+                       : (g32 ? k_refine<REFINE_PLAIN, true, false, 32, 256, false, true>
+                              : k_refine<REFINE_PLAIN, true, false, 8, 256, false, true>);
+        e = run(kp, PS, small, ovf, nullptr, n_items, 256);
+        if (e != cudaSuccess || small >= P.cand_bytes) return e;
         return run(kw, P, wide, nullptr, ovf, n_items, 32 * WIDE_LIST_WARPS);
     }
     auto kern = warm ? (g32 ? pick(k_refine<REFINE_WARM, false, false, 32>, k_refine<REFINE_WARM, true, false, 32>)
