@@ -590,6 +590,7 @@ __device__ __forceinline__ float x_safe_radius(float blocked, float m, double be
 // inside sphere tested; if inside, 1, then 10 per S candidate visited (+7
 // for the projection, +10 per blocker tested), 26 per C candidate (+9 or +6,
 // +10 per blocker), 9 per SAS vertex, 1 final.
+// The counting pass walks every point of an edge.
 template <bool COUNT, bool SAFE>
 __device__ __forceinline__ XEval x_eval(const XView& v, const double* circ, double probe, double band, double x,
                                         double y, double z, XSafe& safe, unsigned long long* ops = nullptr) {
